@@ -404,9 +404,10 @@ int launch_decode(const sqattn_decode_args* a, const DecodePlan& pl, cudaStream_
 
 // ---- kmeans helpers ----------------------------------------------------------------------------------------
 // scratch of the clustering entry points: [max centroid norm per group | flagged count | flagged list | arrival
-// slot per token | offsets per cluster | member list per group | counts per cluster (index_add only)]
+// slot per token | offsets per cluster | member list per group | counts per cluster (index_add only) | cluster counts of
+// the token ranges (reverse_index only)]
 struct KmWorkspace {
-  float* max_cnorm2; int* flagged_count; int* flagged; int* slot; int* offsets; int* members; int* counts;
+  float* max_cnorm2; int* flagged_count; int* flagged; int* slot; int* offsets; int* members; int* counts; int* range_hist;
   int flagged_cap;
   size_t total;
 };
@@ -424,6 +425,7 @@ KmWorkspace km_workspace(void* base, int32_t groups, int32_t num_tokens, int32_t
   w.offsets = reinterpret_cast<int*>(take(gk * sizeof(int)));
   w.members = reinterpret_cast<int*>(take(gt * sizeof(int)));
   w.counts = reinterpret_cast<int*>(take(gk * sizeof(int)));
+  w.range_hist = reinterpret_cast<int*>(take(gk * kSortRanges * sizeof(int)));
   w.total = off;
   return w;
 }
@@ -436,8 +438,10 @@ int km_member_sums(const uint8_t* x, const int32_t* idx, int32_t groups, int32_t
   kmeans_count_kernel<<<elementwise_grid(gt, 256), 256, 0, stream>>>(idx, counts, w.slot, gt, num_tokens, num_centroids);
   kmeans_offsets_kernel<<<groups, 1024, 0, stream>>>(counts, w.offsets, num_centroids);
   kmeans_scatter_kernel<<<elementwise_grid(gt, 256), 256, 0, stream>>>(idx, w.slot, w.offsets, w.members, gt, num_tokens, num_centroids);
-  kmeans_cluster_sum_kernel<D, BF16><<<static_cast<unsigned>((gk * 32 + 255) / 256), 256, 0, stream>>>(
-      x, w.members, w.offsets, counts, sums, gk, num_tokens, num_centroids);
+  SQ_CUDA(cudaMemsetAsync(sums, 0, static_cast<size_t>(gk) * D * sizeof(double), stream));
+  const long long warps = static_cast<long long>(groups) * ((num_tokens + kSumRows - 1) / kSumRows);
+  kmeans_member_sum_kernel<D, BF16><<<static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, stream>>>(
+      x, idx, w.members, sums, groups, num_tokens, num_centroids);
   SQ_CUDA(cudaGetLastError());
   return SQATTN_OK;
 }
@@ -761,13 +765,20 @@ int sqattn_kmeans_reverse_index(const int32_t* idx, int32_t groups, int32_t num_
   if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255))
     return fail(SQATTN_ERR_WORKSPACE, "workspace of %zu bytes (256-byte aligned) required", need);
   const KmWorkspace w = km_workspace(workspace, groups, num_tokens, num_centroids);
-  const long long gt = static_cast<long long>(groups) * num_tokens, gk = static_cast<long long>(groups) * num_centroids;
-  SQ_CUDA(cudaMemsetAsync(w.counts, 0, static_cast<size_t>(gk) * sizeof(int), stream));
-  kmeans_count_kernel<<<elementwise_grid(gt, 256), 256, 0, stream>>>(idx, w.counts, w.slot, gt, num_tokens, num_centroids);
-  kmeans_offsets_kernel<<<groups, 1024, 0, stream>>>(w.counts, w.offsets, num_centroids);
-  kmeans_scatter_kernel<<<elementwise_grid(gt, 256), 256, 0, stream>>>(idx, w.slot, w.offsets, w.members, gt, num_tokens, num_centroids);
-  kmeans_sort_members_kernel<<<static_cast<unsigned>((gk * 32 + 255) / 256), 256, 0, stream>>>(
-      w.members, w.offsets, w.counts, clusters, cluster_size, gk, num_tokens, num_centroids, max_cluster_size);
+  // a range is a multiple of 32 tokens, at least 256 of them
+  int per_range = ((num_tokens + kSortRanges - 1) / kSortRanges + 31) / 32 * 32;
+  if (per_range < 256) per_range = 256;
+  const dim3 ranges((num_tokens + per_range - 1) / per_range, groups);
+  const int smem = (num_centroids < kSortClusters ? num_centroids : kSortClusters) * static_cast<int>(sizeof(int));
+  SQ_CUDA(cudaFuncSetAttribute(kmeans_range_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  SQ_CUDA(cudaFuncSetAttribute(kmeans_range_emit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  for (int c0 = 0; c0 < num_centroids; c0 += kSortClusters)
+    kmeans_range_count_kernel<<<ranges, 32, smem, stream>>>(idx, w.range_hist, num_tokens, num_centroids, per_range, c0,
+                                                            num_centroids - c0 < kSortClusters ? num_centroids - c0 : kSortClusters);
+  kmeans_range_scan_kernel<<<dim3((num_centroids + 255) / 256, groups), 256, 0, stream>>>(w.range_hist, cluster_size, ranges.x, num_centroids);
+  for (int c0 = 0; c0 < num_centroids; c0 += kSortClusters)
+    kmeans_range_emit_kernel<<<ranges, 32, smem, stream>>>(idx, w.range_hist, clusters, num_tokens, num_centroids, per_range, max_cluster_size, c0,
+                                                           num_centroids - c0 < kSortClusters ? num_centroids - c0 : kSortClusters);
   SQ_CUDA(cudaGetLastError());
   return SQATTN_OK;
 }

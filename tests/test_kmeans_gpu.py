@@ -108,3 +108,28 @@ def test_clustered_retrieval_ragged_decode():
             assert (out[i, h * groups:(h + 1) * groups].float() - ro[0].float()).abs().max().item() < 6e-2
             ro = so.decode(qh, kq, vq, output_dtype=torch.bfloat16, center_k=False, mask_tail=True)
             assert (out16[i, h * groups:(h + 1) * groups].float() - ro[0].float()).abs().max().item() < 2e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("t,d", [(1, 128), (63, 128), (64, 64), (65, 128), (257, 128), (5000, 64), (20000, 128)])
+def test_member_sums_and_lists_with_uneven_clusters(dtype, t, d):
+    """Sums and sorted lists where they are cut into ranges: one cluster holds half of the tokens, others one or none.
+    The fp64 sum of 16-bit values is exact, so the sums are compared exactly."""
+    from longcontext_sqattn_paddle_b200.cache_hub import kmeans as km
+    g, k = 2, 96
+    gen = torch.Generator().manual_seed(t + d)
+    idx = torch.randint(0, k - 5, (g, t), generator=gen, dtype=torch.int32)      # the last clusters stay empty
+    idx[torch.rand(g, t, generator=gen) < 0.5] = 7
+    val = torch.randn(g, t, d, generator=gen).to(dtype)
+    val[0, 0, 0], val[1, t - 1, 1] = 0.0, 6e-8                                    # zero and a subnormal of the half type
+    sums = torch.zeros(g, k, d, dtype=torch.float64)
+    sums.scatter_add_(1, idx.long()[..., None].expand(-1, -1, d), val.double())
+    got = km.index_add(val.cuda(), idx.cuda(), k)
+    assert torch.equal(got.cpu(), sums.float().to(dtype))
+    n = torch.stack([torch.bincount(r.long(), minlength=k) for r in idx])
+    width = int(n.max())
+    lists, size = km.reverse_index(idx.cuda(), k, width)
+    assert torch.equal(size.cpu().long(), n)
+    for b in range(g):
+        for c in range(k):
+            assert torch.equal(lists[b, c, :n[b, c]].cpu().long(), (idx[b] == c).nonzero()[:, 0])
