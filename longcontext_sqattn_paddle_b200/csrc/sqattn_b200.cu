@@ -13,6 +13,7 @@
 #include "prefill.cuh"
 #include "prep.cuh"
 #include "retrieval.cuh"
+#include "window_hist_tc.cuh"
 #include "window_search.cuh"
 
 using namespace sq;
@@ -462,6 +463,24 @@ int km_launch_assign(const void* data, const void* centroids, int32_t dtype, int
   SQ_CUDA(cudaFuncSetAttribute(kmeans_assign_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
   const dim3 grid((num_tokens + kKtTokens - 1) / kKtTokens, groups);
   kmeans_assign_tc_kernel<D><<<grid, 320, L::kTotal, stream>>>(td, tc, p);
+  SQ_CUDA(cudaGetLastError());
+  return SQATTN_OK;
+}
+
+// ---- window calibration ------------------------------------------------------------------------------------
+template <int D>
+int launch_window_hist_tc(const WindowHistParams& p, int dtype, cudaStream_t stream) {
+  CUtensorMap tq, tk;
+  int rc;
+  const int hkv = p.hq / p.groups;
+  const int64_t sh = static_cast<int64_t>(p.n) * D;
+  if ((rc = make_tmap_bhnd(&tq, p.q, dtype, sh * p.hq, sh, D, 1, p.hq, p.n, D, kWtRows, "q"))) return rc;
+  if ((rc = make_tmap_bhnd(&tk, p.k, dtype, sh * hkv, sh, D, 1, hkv, p.n, D, kWtKeys, "k"))) return rc;
+  size_t smem = WindowTcSmem<D>::total(p.nbins);
+  if (smem < 116 * 1024) smem = 116 * 1024;   // one CTA per SM: each one allocates all of the tensor memory
+  SQ_CUDA(cudaFuncSetAttribute(window_hist_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  const unsigned grid = static_cast<unsigned>((p.n + kWtRows - 1) / kWtRows) * p.hq;
+  window_hist_tc_kernel<D><<<grid, 320, smem, stream>>>(tq, tk, p, dtype == SQATTN_BF16);
   SQ_CUDA(cudaGetLastError());
   return SQATTN_OK;
 }
@@ -933,8 +952,14 @@ int sqattn_window_histogram(const void* q, const void* k, int32_t dtype, int32_t
   p.hq = num_q_heads; p.groups = num_q_heads / num_kv_heads; p.n = seq_len; p.d = head_dim; p.nbins = num_bins;
   p.sink = sink; p.relative = relative; p.scale = static_cast<float>(1.0 / sqrt(static_cast<double>(head_dim)));
   const bool bf16 = dtype == SQATTN_BF16;
+  // Relative distances go to the tcgen05 kernel while the rows' histograms fit into shared memory and a bin is no finer
+  // than its edge arithmetic assumes.  Absolute distances have a bin per key, which that kernel's runs gain nothing from.
+  if ((head_dim == 64 || head_dim == 128) && relative && num_bins <= kWtMaxBins &&
+      seq_len <= static_cast<long long>(kWtKeysPerBin) * num_bins && !((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k)) & 15) &&
+      static_cast<long long>((seq_len + kWtRows - 1) / kWtRows) * num_q_heads <= 0x7fffffffll)
+    return head_dim == 128 ? launch_window_hist_tc<128>(p, dtype, stream) : launch_window_hist_tc<64>(p, dtype, stream);
   if (head_dim == 64 || head_dim == 128) {
-    // tensor-core kernel: Q tile + two K tiles (rows padded by 8 elements) + the block histogram
+    // mma.sync kernel: Q tile + two K tiles (rows padded by 8 elements) + the block histogram
     const size_t smem = static_cast<size_t>(3) * 64 * (head_dim + 8) * 2 + static_cast<size_t>(num_bins) * sizeof(float);
     if (smem > 220 * 1024) return fail(SQATTN_ERR_UNSUPPORTED, "too many bins (%d)", num_bins);
     const dim3 grid((seq_len + kWhRows - 1) / kWhRows, num_q_heads);

@@ -49,3 +49,21 @@ def test_histogram_kernel_matches_dense_map(relative, sink):
 
     b8, b4, windows = ws.calibrate_windows([(q.cuda(), k.cuda())], Args(), max_len=n)
     assert len(windows) == hq and b8 <= b4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,d,bins,sink", [(1, 128, 200, 0), (5, 64, 7, 256), (127, 128, 1, 0), (128, 128, 100, 5), (129, 128, 200, 0),
+                                           (257, 64, 256, 256), (1000, 128, 3, 130), (2311, 128, 200, 256), (2500, 64, 100, 77)])
+def test_relative_histogram_at_tile_and_bin_edges(n, d, bins, sink):
+    """Rows that end inside a tile, sinks that do, bins narrower and wider than the kernel's key groups.  All weights are
+    positive, so a bin's relative error is at most that of a pair: 2^-22 of the exponential plus the rounding of an fp32
+    score of magnitude <= 40 summed over 128 products (3e-6 each way)."""
+    from longcontext_sqattn_paddle_b200.sqattn import window_search as ws
+    for dtype in (torch.bfloat16, torch.float16):
+        g = torch.Generator().manual_seed(n)
+        q, k = torch.randn(4, n, d, generator=g).to(dtype), torch.randn(2, n, d, generator=g).to(dtype)
+        k[..., 5::32] *= 8.0
+        hist = ws.attention_histograms(q.cuda(), k.cuda(), relative=True, num_bins=bins, sink_len=sink).cpu().numpy()
+        a = wo.attention_map(q, k)
+        for h in range(4):
+            np.testing.assert_allclose(hist[h], wo.relative_histogram_with_sink(a[h], bins, sink), rtol=5e-5, atol=1e-30)
