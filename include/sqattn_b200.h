@@ -206,6 +206,12 @@ typedef struct {
 size_t sqattn_decode_workspace_bytes(const sqattn_decode_args* args);
 int sqattn_decode(const sqattn_decode_args* args, sqattn_stream_t stream);
 
+/* Decode over centred keys, K - mean over the kv_len keys (attn_unified with its defaults, attn_triton_decode.py:268-269),
+ * in one pass over K and V: the mean, rounded to the keys' type, only shifts the scores and the LSE.  Needs a workspace
+ * of its own size; kv_lens, kv_lens_device, gather, peer, partial_o and p_fp8 are rejected (SQATTN_ERR_INVALID_ARG). */
+size_t sqattn_decode_centered_workspace_bytes(const sqattn_decode_args* args);
+int sqattn_decode_centered(const sqattn_decode_args* args, sqattn_stream_t stream);
+
 /* No counterpart in the reference.  Same computation and results as sqattn_decode, for callers that cannot
  * give it a workspace because they may not allocate device memory where they call from: code running inside
  * a framework's memory-planned region or a serving loop with a frozen memory pool, where a cudaMalloc (or a

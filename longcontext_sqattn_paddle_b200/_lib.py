@@ -104,6 +104,8 @@ SYMBOLS = [
                                        C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
     ("sqattn_decode_workspace_bytes", C.c_size_t, [C.POINTER(DecodeArgs)]),
     ("sqattn_decode", C.c_int, [C.POINTER(DecodeArgs), C.c_void_p]),
+    ("sqattn_decode_centered_workspace_bytes", C.c_size_t, [C.POINTER(DecodeArgs)]),
+    ("sqattn_decode_centered", C.c_int, [C.POINTER(DecodeArgs), C.c_void_p]),
     ("sqattn_decode_static_scratch", C.c_int, [C.POINTER(DecodeArgs), C.c_void_p]),
     ("sqattn_decode_merge", C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_int64, C.c_int32, C.c_void_p, C.c_int32,
                                       C.c_void_p, C.c_void_p]),

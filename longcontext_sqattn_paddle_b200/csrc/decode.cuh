@@ -9,6 +9,8 @@
 //   warps 0..3  16 keys of every tile each: S = q K^T and O += P V on mma.sync m16n8k16 (query heads padded
 //               to the 16-row M dimension), warp-shuffle row max / sum, private online-softmax state;
 //               the four states are merged through shared memory at the end of the item.
+//   warps 6..9  only where the caller wants the keys centred (kColSum): column sums of the same K tiles, so that the
+//               mean costs no pass of its own (centring is a shift of the scores; see decode_center_merge_kernel).
 // A second kernel merges the per-range partials (base-2 LSE).
 #pragma once
 #include <cuda.h>
@@ -42,6 +44,7 @@ struct DecodeParams {
   const uint8_t* const* gather_v;
   long long gather_row_stride;  // elements
   int gather_cap;
+  float* part_ksum;  // kColSum: column sums of the item's keys, [items, Hkv, D]
 };
 
 // 16-byte asynchronous copy global -> shared, and an arrival on `bar` once all of this thread's copies have landed
@@ -86,7 +89,8 @@ struct DecodeSmem {
   static constexpr int kStageBytes = 2 * kTileBytes;             // K then V
   static constexpr int kBarOff = kDecStages * kStageBytes;       // full[3], empty[3]
   static constexpr int kMiscOff = kBarOff + 8 * 2 * kDecStages;  // abort flag
-  static constexpr int kTotal = kMiscOff + 16;
+  static constexpr int kSumOff = kMiscOff + 16;                  // kColSum: the four summing warps' columns [4][D] fp32
+  static constexpr int kTotal = kSumOff + 4 * D * 4;
   static constexpr int kDynBytes = kTotal + 1024;
   // the merge scratch (4 warps x (16 x D fp32 + 32 floats)) reuses the tile ring
   static_assert(4 * (16 * D + 32) * 4 <= kDecStages * kStageBytes, "merge scratch must fit in the ring");
@@ -103,8 +107,10 @@ __device__ __forceinline__ uint32_t tile_off(int key, int chunk) {
 __device__ unsigned long long g_dec_first = ~0ull, g_dec_last = 0ull;
 #endif
 
-template <int D, bool BF16>
-__global__ void __launch_bounds__(192, 2)
+constexpr int decode_threads(bool col_sum) { return col_sum ? 320 : 192; }
+
+template <int D, bool BF16, bool kColSum>
+__global__ void __launch_bounds__(decode_threads(kColSum), kColSum ? 1 : 2)
 decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
               const __grid_constant__ DecodeParams p) {
   using L = DecodeSmem<D>;
@@ -157,13 +163,52 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     *cta_abort = 0;
     // a stage is full after the producer's one arrival + its bytes (TMA), or after the copies of all 64 lanes of the
     // two copying warps (index list)
-    for (int i = 0; i < kDecStages; ++i) { mbar_init(bar_full + 8 * i, p.gather_idx ? 64 : 1); mbar_init(bar_empty + 8 * i, 4); }
+    for (int i = 0; i < kDecStages; ++i) { mbar_init(bar_full + 8 * i, p.gather_idx ? 64 : 1); mbar_init(bar_empty + 8 * i, kColSum ? 8 : 4); }
     fence_barrier_init();
     fence_proxy_async();
   }
   __syncthreads();
 
-  if (warp >= 4 && p.gather_idx) {
+  if (kColSum && warp >= 6) {
+    // ---- column sums: a warp takes 16 rows of every tile, D / 8 lanes per row with 16-byte reads
+    constexpr int kLanesPerRow = D / 8, kRows = 32 / kLanesPerRow;
+    const int sw = warp - 6, c = lane % kLanesPerRow, rsel = lane / kLanesPerRow;
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    bool ok = true;
+    for (int t = 0; ok && t < ntiles; ++t) {
+      const int st = t % kDecStages;
+      ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * st, (t / kDecStages) & 1, cta_abort, 203));
+      if (!ok) break;
+      const uint8_t* k_tile = smem + st * L::kStageBytes;
+      const int key0 = key_begin + t * kDecTile;
+      uint4 v[16 / kRows];
+#pragma unroll
+      for (int u = 0; u < 16 / kRows; ++u) {
+        const int r = sw * 16 + u * kRows + rsel;
+        v[u] = *reinterpret_cast<const uint4*>(k_tile + tile_off(r, c));
+        if (key0 + r >= key_end) v[u] = make_uint4(0u, 0u, 0u, 0u);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_empty + 8 * st);
+#pragma unroll
+      for (int u = 0; u < 16 / kRows; ++u) {
+        float f[8];
+        unpack8<BF16>(v[u], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += f[e];
+      }
+    }
+    float* col = reinterpret_cast<float*>(smem + L::kSumOff);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      for (int o = kLanesPerRow; o < 32; o <<= 1) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+      if (rsel == 0) col[sw * D + c * 8 + e] = acc[e];
+    }
+    asm volatile("bar.sync 2, 128;" ::: "memory");
+    const int d = threadIdx.x - 192;
+    if (ok && d < D)
+      p.part_ksum[(static_cast<long long>(item) * p.hkv + kvh) * D + d] = (col[d] + col[D + d]) + (col[2 * D + d] + col[3 * D + d]);
+  } else if (warp >= 4 && p.gather_idx) {
     const int half = warp - 4;   // warps 4 and 5 copy the even and the odd row groups of every tile
     const long long grp = static_cast<long long>(bi) * p.hkv + kvh;
     const int* idx = p.gather_idx + grp * p.gather_cap;
@@ -518,6 +563,71 @@ __global__ void __launch_bounds__(128 * kMergeGroups) decode_merge_kernel(const 
     else if (p.o_dtype) reinterpret_cast<uint16_t*>(p.o)[off] = from_f32<true>(val);
     else reinterpret_cast<uint16_t*>(p.o)[off] = from_f32<false>(val);
     if (col == 0 && p.lse) p.lse[row] = lse;
+  }
+}
+
+// ---- decode over centred keys --------------------------------------------------------------------------------
+// The launcher with the reference's defaults attends K' = K - mean(K) (attn_triton_decode.py:268-269).  For one query
+// q . k' = q . k - c with c = q . mean, a shift of every score, so K' is never formed: the decode kernel runs on K and
+// adds up its columns on the way, and this merge takes c off the LSE and gives the zero keys that pad the last 64-key
+// tile (score 0 in K', hence c here, value 0) their share.  Forming K' took a fp32 copy, a mean, a subtraction and a
+// second pass over K: 169 us a call at 32000 keys x 4 heads, 34 us (most of it the host's) with one pass over 65.5 MB.
+struct CenterMergeParams {
+  MergeParams m;           // ragged form
+  const float* part_ksum;  // [items, Hkv, D]
+  const uint8_t* q;
+  long long q_sb, q_sh;    // elements
+  int hkv, groups, q_is_scaled, reference_tail;
+  float sm_scale;
+  int lens[kDecMaxBatch];
+};
+
+template <bool BF16>
+__global__ void __launch_bounds__(128 * kMergeGroups) decode_center_merge_kernel(const __grid_constant__ CenterMergeParams p) {
+  __shared__ MergeScratch sm;
+  __shared__ float c_s[4];
+  griddep_launch();
+  griddep_wait();  // the partials come from the kernel launched just before
+  const long long row = blockIdx.x;  // b*hq + h
+  const int b = static_cast<int>(row / p.m.hq), h = static_cast<int>(row % p.m.hq), kvh = h / p.groups;
+  const int first = p.m.item_prefix[b], count = p.m.item_prefix[b + 1] - first, d = p.m.d;
+  const int tid = threadIdx.x, col = tid % 128, grp = tid / 128;
+  // c = (q as the decode kernel uses it) . (mean rounded to the keys' type, as the reference subtracts it)
+  float s = 0.f;
+  if (col < d)
+    for (int i = grp; i < count; i += kMergeGroups) s += p.part_ksum[(static_cast<long long>(first + i) * p.hkv + kvh) * d + col];
+  sm.red[grp][col] = s;
+  __syncthreads();
+  if (grp == 0) {
+    float prod = 0.f;
+    if (col < d) {
+      const float sum = (sm.red[0][col] + sm.red[1][col]) + (sm.red[2][col] + sm.red[3][col]);
+      const float mean = to_f32<BF16>(from_f32<BF16>(sum / static_cast<float>(p.lens[b])));
+      float qv = to_f32<BF16>(*reinterpret_cast<const uint16_t*>(p.q + 2 * (b * p.q_sb + h * p.q_sh + col)));
+      if (!p.q_is_scaled) qv = to_f32<BF16>(from_f32<BF16>(qv * p.sm_scale));
+      prod = qv * mean;
+    }
+    for (int o = 16; o > 0; o >>= 1) prod += __shfl_xor_sync(0xffffffffu, prod, o);
+    if ((tid & 31) == 0) c_s[tid >> 5] = prod;
+  }
+  __syncthreads();
+  const float c = (c_s[0] + c_s[1]) + (c_s[2] + c_s[3]);
+  float val, lse;
+  merge_row_partials(p.m.part_o, p.m.part_lse, static_cast<long long>(first) * p.m.hq + h, p.m.hq, count, d, sm, val, lse);
+  const int len = p.lens[b], pad = p.reference_tail ? (len + kDecTile - 1) / kDecTile * kDecTile - len : 0;
+  if (pad > 0) {
+    const float lt = c + log2f(static_cast<float>(pad)), top = fmaxf(lse, lt);
+    const float keys = exp2f(lse - top), all = keys + exp2f(lt - top);
+    val *= keys / all;
+    lse = top + log2f(all);
+  }
+  lse -= c;
+  if (!(fabsf(c) <= 3.0e38f)) val = lse = __int_as_float(0x7fc00000);  // an infinity or a NaN among the keys: K' is NaN
+  if (tid < d) {
+    const long long off = b * p.m.o_sb + h * p.m.o_sh + tid;
+    if (p.m.o_dtype) reinterpret_cast<uint16_t*>(p.m.o)[off] = from_f32<true>(val);
+    else reinterpret_cast<uint16_t*>(p.m.o)[off] = from_f32<false>(val);
+    if (tid == 0 && p.m.lse) p.m.lse[row] = lse;
   }
 }
 

@@ -335,7 +335,12 @@ int fill_peer_params(const sqattn_peer_merge_args* a, PeerMergeParams* p) {
   return SQATTN_OK;
 }
 
-template <int D, bool BF16>
+// column sums of the keys of every work item (centred decode)
+size_t decode_ksum_bytes(const sqattn_decode_args* a, const DecodePlan& pl) {
+  return static_cast<size_t>(pl.total_items > 0 ? pl.total_items : 1) * a->num_kv_heads * a->head_dim * 4;
+}
+
+template <int D, bool BF16, bool kCentered = false>
 int launch_decode(const sqattn_decode_args* a, const DecodePlan& pl, cudaStream_t stream) {
   CUtensorMap tk, tv;
   int rc;
@@ -362,14 +367,15 @@ int launch_decode(const sqattn_decode_args* a, const DecodePlan& pl, cudaStream_
   p.part_o = reinterpret_cast<float*>(ws);
   p.part_lse = reinterpret_cast<float*>(ws + align_up(rows * D * 4, 256));
   p.batch = a->batch; p.hq = a->num_q_heads; p.hkv = a->num_kv_heads; p.groups = a->num_q_heads / a->num_kv_heads; p.d = D;
-  p.chunk = pl.chunk; p.p_fp8 = a->p_fp8; p.q_is_scaled = a->q_is_scaled; p.reference_tail = a->reference_tail;
+  p.chunk = pl.chunk; p.p_fp8 = a->p_fp8; p.q_is_scaled = a->q_is_scaled; p.reference_tail = kCentered ? 0 : a->reference_tail;
   p.sm_scale = static_cast<float>(sm_scale_log2(D, a->head_dim_og));
   memcpy(p.lens, pl.lens, sizeof(int) * a->batch);
   p.lens_dev = a->kv_lens_device;
   memcpy(p.item_prefix, pl.prefix, sizeof(int) * (a->batch + 1));
   using L = DecodeSmem<D>;
   // a function attribute belongs to the current device: set on every call, like the prefill launch does
-  SQ_CUDA(cudaFuncSetAttribute(decode_kernel<D, BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynBytes));
+  SQ_CUDA(cudaFuncSetAttribute(decode_kernel<D, BF16, kCentered>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynBytes));
+  if (kCentered) p.part_ksum = reinterpret_cast<float*>(ws + decode_ws_bytes(a, pl));
   PeerMergeParams pm;
   if (a->peer) {  // checked before anything is launched
     if ((rc = fill_peer_params(a->peer, &pm))) return rc;
@@ -379,7 +385,7 @@ int launch_decode(const sqattn_decode_args* a, const DecodePlan& pl, cudaStream_
   }
   if (pl.total_items > 0) {
     dim3 grid(pl.total_items, a->num_kv_heads);
-    SQ_CUDA(launch_overlapped(2, decode_kernel<D, BF16>, grid, dim3(192), L::kDynBytes, stream, tk, tv, p));
+    SQ_CUDA(launch_overlapped(2, decode_kernel<D, BF16, kCentered>, grid, dim3(decode_threads(kCentered)), L::kDynBytes, stream, tk, tv, p));
   }
 
   if (a->peer) {
@@ -399,7 +405,17 @@ int launch_decode(const sqattn_decode_args* a, const DecodePlan& pl, cudaStream_
   } else {
     m.o = a->o.ptr; m.lse = a->lse; m.o_dtype = a->o_dtype; m.o_sb = a->o.stride_b; m.o_sh = a->o.stride_h;
   }
-  SQ_CUDA(launch_overlapped(1, decode_merge_kernel, dim3(static_cast<unsigned>(m.rows)), dim3(128 * kMergeGroups), 0, stream, m));
+  if constexpr (kCentered) {
+    CenterMergeParams cm;
+    memset(&cm, 0, sizeof(cm));
+    cm.m = m; cm.part_ksum = p.part_ksum;
+    cm.q = p.q; cm.q_sb = p.q_sb; cm.q_sh = p.q_sh;
+    cm.hkv = p.hkv; cm.groups = p.groups; cm.q_is_scaled = p.q_is_scaled; cm.reference_tail = a->reference_tail; cm.sm_scale = p.sm_scale;
+    memcpy(cm.lens, pl.lens, sizeof(int) * a->batch);
+    SQ_CUDA(launch_overlapped(1, decode_center_merge_kernel<BF16>, dim3(static_cast<unsigned>(m.rows)), dim3(128 * kMergeGroups), 0, stream, cm));
+  } else {
+    SQ_CUDA(launch_overlapped(1, decode_merge_kernel, dim3(static_cast<unsigned>(m.rows)), dim3(128 * kMergeGroups), 0, stream, m));
+  }
   return SQATTN_OK;
 }
 
@@ -615,8 +631,7 @@ size_t sqattn_decode_workspace_bytes(const sqattn_decode_args* args) {
   return decode_ws_bytes(args, pl);
 }
 
-int sqattn_decode(const sqattn_decode_args* a, sqattn_stream_t stream_) {
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+static int decode_impl(const sqattn_decode_args* a, cudaStream_t stream, bool centered) {
   DecodePlan pl;
   int rc = plan_decode(a, &pl);
   if (rc) return rc;
@@ -625,12 +640,41 @@ int sqattn_decode(const sqattn_decode_args* a, sqattn_stream_t stream_) {
   if (a->partial_o && !a->partial_lse) return fail(SQATTN_ERR_INVALID_ARG, "partial_lse missing");
   if (!a->gather && (!aligned16(a->k) || !aligned16(a->v))) return fail(SQATTN_ERR_INVALID_ARG, "k/v need 16-byte alignment");
   if ((reinterpret_cast<uintptr_t>(a->q.ptr) % 4) || (a->q.stride_h % 2) || (a->q.stride_b % 2)) return fail(SQATTN_ERR_INVALID_ARG, "q needs 4-byte alignment");
-  const size_t need = decode_ws_bytes(a, pl);
+  const size_t need = decode_ws_bytes(a, pl) + (centered ? decode_ksum_bytes(a, pl) : 0);
   if (!a->workspace || a->workspace_bytes < need || (reinterpret_cast<uintptr_t>(a->workspace) % 256))
     return fail(SQATTN_ERR_WORKSPACE, "workspace of %zu bytes (256-byte aligned) required", need);
   const bool bf16 = a->dtype == SQATTN_BF16;
+  if (centered) {
+    if (a->head_dim == 128) return bf16 ? launch_decode<128, true, true>(a, pl, stream) : launch_decode<128, false, true>(a, pl, stream);
+    return bf16 ? launch_decode<64, true, true>(a, pl, stream) : launch_decode<64, false, true>(a, pl, stream);
+  }
   if (a->head_dim == 128) return bf16 ? launch_decode<128, true>(a, pl, stream) : launch_decode<128, false>(a, pl, stream);
   return bf16 ? launch_decode<64, true>(a, pl, stream) : launch_decode<64, false>(a, pl, stream);
+}
+
+int sqattn_decode(const sqattn_decode_args* a, sqattn_stream_t stream) {
+  return decode_impl(a, reinterpret_cast<cudaStream_t>(stream), false);
+}
+
+// what sqattn_decode_centered takes: every key of the sequences counts for the mean, so no lengths of its own, and an FP8 P
+// depends on the running maximum of the centred scores
+static int centered_check(const sqattn_decode_args* a) {
+  if (!a) return fail(SQATTN_ERR_INVALID_ARG, "args is null");
+  if (a->kv_lens || a->kv_lens_device || a->gather || a->peer || a->partial_o || a->p_fp8)
+    return fail(SQATTN_ERR_INVALID_ARG, "centred decode: no kv_lens, gather, peer, partial output or FP8 P");
+  if (a->kv_len <= 0) return fail(SQATTN_ERR_INVALID_ARG, "centred decode: kv_len %d", a->kv_len);
+  return SQATTN_OK;
+}
+
+size_t sqattn_decode_centered_workspace_bytes(const sqattn_decode_args* a) {
+  DecodePlan pl;
+  if (centered_check(a) || plan_decode(a, &pl)) return 0;
+  return decode_ws_bytes(a, pl) + decode_ksum_bytes(a, pl);
+}
+
+int sqattn_decode_centered(const sqattn_decode_args* a, sqattn_stream_t stream) {
+  const int rc = centered_check(a);
+  return rc ? rc : decode_impl(a, reinterpret_cast<cudaStream_t>(stream), true);
 }
 
 int sqattn_decode_merge(const float* partial_o, const float* partial_lse, int32_t num_parts, int64_t rows,

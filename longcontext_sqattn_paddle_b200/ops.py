@@ -254,6 +254,36 @@ def decode(q, k, v, *, layout: str = "HND", out_dtype=torch.float16, return_lse:
     return (out, lse) if return_lse else out
 
 
+def tma_ready(t: torch.Tensor, layout: str) -> bool:
+    """The kernels can read ``t`` where it lies: 16-byte aligned rows, no broadcast dimension."""
+    b, h, n, d = _shape(t, layout)
+    v = _view(t, layout) if t.stride(-1) == 1 else None
+    return v is not None and t.data_ptr() % 16 == 0 and all(
+        s % 8 == 0 and (s > 0 or ext == 1) for s, ext in ((v.stride_b, b), (v.stride_h, h), (v.stride_n, n)))
+
+
+def decode_centered(q, k, v, *, layout: str = "HND", out_dtype=torch.float16, return_lse: bool = False,
+                    reference_tail: bool = False, head_dim_og: int = 0):
+    """sqattn_decode_centered: ``decode`` over K minus its mean over all the keys given, without forming it."""
+    _require_cuda(q, k, v)
+    poll_device_status(q.device)
+    b, hq, one, d = _shape(q, layout)
+    assert one == 1
+    _, hkv, cap, _ = _shape(k, layout)
+    a = L.DecodeArgs()
+    out = torch.empty(q.shape, dtype=out_dtype, device=q.device)
+    lse = torch.empty(b, hq, 1, dtype=torch.float32, device=q.device) if return_lse else None
+    a.q, a.k, a.v, a.o = _view(q, layout), _view(k, layout), _view(v, layout), _view(out, layout)
+    a.batch, a.num_q_heads, a.num_kv_heads, a.head_dim, a.head_dim_og = b, hq, hkv, d, int(head_dim_og)
+    a.kv_len, a.dtype, a.o_dtype, a.reference_tail = cap, _dt(k.dtype), _dt(out_dtype), int(reference_tail)
+    a.lse = lse.data_ptr() if return_lse else None
+    need = L.lib.sqattn_decode_centered_workspace_bytes(C.byref(a))
+    ws = _workspace(need, q.device)    # 0: the plan was rejected, the entry point reports why
+    a.workspace, a.workspace_bytes = (ws.data_ptr() if ws is not None else None), need
+    L.check(L.lib.sqattn_decode_centered(C.byref(a), _stream()))
+    return (out, lse) if return_lse else out
+
+
 def decode_gather(q, idx, counts, k_rows, v_rows, row_stride: int, kv_dtype, *, out_dtype=torch.float16,
                   p_fp8: bool = False, q_is_scaled: bool = False, num_kv_heads: int = 1):
     """sqattn_decode over listed rows (sqattn_decode_args.gather): q [B,Hq,1,D]; key j of (sequence b, KV head h) is row

@@ -92,9 +92,18 @@ def attn_causal(q, k, v, tensor_layout="HND", output_dtype=torch.float16, return
 def attn_unified(q, k, v, tensor_layout="HND", output_dtype=torch.float16, return_lse=False, is_P_fp8_quant=False,
                  center_k=True, kv_lens=None):
     """qo_len == 1 -> split-KV decode, otherwise dense causal prefill.  The reference subtracts the sequence
-    mean from K on every call (attn_triton_decode.py:268-269); ``center_k=False`` skips that pass, which does
-    not change a single-query softmax."""
+    mean from K on every call (attn_triton_decode.py:268-269); ``center_k=False`` skips that, which does
+    not change a single-query softmax.  A single query over whole caches takes the mean along the way
+    (ops.decode_centered: 32000 keys x 4 heads in one pass over K and V instead of four over K and one over both);
+    lengths of their own (the mean covers all of K), an FP8 P (its rounding follows the running maximum of the
+    centred scores), keys that the kernel cannot read where they lie (the difference is a fresh tensor) and a
+    head_dim that is padded anyway go through the centred copy."""
     seq_dim = 1 if tensor_layout == "NHD" else 2
+    if (center_k and kv_lens is None and not is_P_fp8_quant and tensor_layout in ("HND", "NHD") and q.shape[seq_dim] == 1
+            and q.dim() == k.dim() == 4 and q.shape[-1] in (64, 128) and q.dtype == k.dtype == v.dtype
+            and k.dtype in (torch.float16, torch.bfloat16) and k.is_cuda and k.numel() and ops.tma_ready(k, tensor_layout)):
+        return ops.decode_centered(q, k, v, layout=tensor_layout, out_dtype=output_dtype, return_lse=return_lse,
+                                   reference_tail=True)
     if center_k:
         km = k.float().mean(dim=seq_dim, keepdim=True).to(k.dtype)
         k = k - km

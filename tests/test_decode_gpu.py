@@ -146,3 +146,56 @@ def test_decode_over_listed_rows_equals_decode_over_packed_copies(dtype, fp8, d)
     ref = ops.decode(q, k_sel, v_sel, out_dtype=dtype, p_fp8=fp8, kv_len=cap, kv_lens_device=cnt)
     assert torch.isfinite(out.float()).all()
     assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("layout", ["HND", "NHD", "strided"])
+@pytest.mark.parametrize("b,hq,hkv,L,d", [(1, 28, 4, 1, 128), (2, 8, 1, 63, 64), (1, 28, 4, 64, 128), (3, 32, 8, 65, 128),
+                                          (1, 16, 1, 257, 64), (2, 28, 4, 5003, 128), (1, 28, 4, 40000, 128)])
+def test_centred_decode_in_one_pass(dtype, layout, b, hq, hkv, L, d):
+    """attn_unified without a centred copy of K against the definition in fp64: keys minus their rounded mean (not
+    rounded again), the last 64-key tile padded with zero keys.  Keys with an offset that the mean takes off again.
+    O: P and the result are rounded to 16 bits, 2 * 2^-9 (bf16) or 2^-11 (f16) of values up to 5; LSE: fp32 sums of 128
+    products of scores up to 100, 1e-3.  The path over a centred copy (kv_lens given) rounds every key as well."""
+    from longcontext_sqattn_paddle_b200.sqattn import attn_unified
+    q, k, v = _rand((b, hq, 1, d), L, dtype), _rand((b, hkv, L, d), L + 1, dtype), _rand((b, hkv, L, d), L + 2, dtype)
+    k[..., 3::32] += 2.0
+    qs = (q.float() * np.float32(1.0 / d ** 0.5 * 1.44269504)).to(dtype).double()
+    kc = k.double() - k.double().mean(dim=2, keepdim=True).to(dtype).double()
+    pad = -L % 64
+    kc, vd = (torch.cat([t, torch.zeros(b, hkv, pad, d, dtype=torch.float64)], 2).repeat_interleave(hq // hkv, 1)
+              for t in (kc, v.double()))
+    s = qs @ kc.transpose(2, 3)
+    ref, rlse = torch.softmax(s * np.log(2.0), -1) @ vd, torch.logsumexp(s * np.log(2.0), -1) / np.log(2.0)
+    if layout == "NHD":
+        args = [t.transpose(1, 2).contiguous().cuda() for t in (q, k, v)]
+    elif layout == "strided":   # K and V as halves of one wider row, more rows than are attended
+        kv = torch.cat([torch.stack([k, v], 3), torch.full((b, hkv, 5, 2, d), float("nan"), dtype=dtype)], 2).cuda()
+        args = [q.cuda(), kv[:, :, :L, 0], kv[:, :, :L, 1]]
+    else:
+        args = [t.cuda() for t in (q, k, v)]
+    lay = "NHD" if layout == "NHD" else "HND"
+    o, lse = attn_unified(*args, lay, dtype, True)
+    assert (lse.cpu().double() - rlse.view(b, hq, 1)).abs().max().item() < 1e-3
+    o = (o.transpose(1, 2) if layout == "NHD" else o).cpu().double()
+    assert (o - ref).abs().max().item() < (2e-2 if dtype == torch.bfloat16 else 5e-3)
+    o2, lse2 = attn_unified(*args, lay, dtype, True, kv_lens=[L] * b)
+    tol = 0.3 if dtype == torch.bfloat16 else 4e-2   # a rounded key: 2^-9 of values up to 40 summed over the row, both ways
+    assert (lse.cpu() - lse2.cpu()).abs().max().item() < tol
+
+
+def test_centred_decode_keeps_the_copy_where_it_has_to():
+    """Broadcast and misaligned keys, an FP8 P, and an infinite key (the centred keys are NaN either way)."""
+    from longcontext_sqattn_paddle_b200.sqattn import attn_unified
+    dtype = torch.bfloat16
+    q, k, v = (_rand(s, i, dtype).cuda() for i, s in enumerate([(2, 8, 1, 128), (1, 2, 300, 128), (2, 2, 300, 128)]))
+    full = attn_unified(q, k.expand(2, -1, -1, -1).contiguous(), v, "HND", dtype)
+    wide = torch.zeros(2, 2, 300, 132, dtype=dtype, device="cuda")
+    wide[..., 1:129] = k
+    for kk in (k.expand(2, -1, -1, -1), wide[..., 1:129]):
+        assert (attn_unified(q, kk, v, "HND", dtype).float() - full.float()).abs().max().item() < 3e-2
+    assert torch.isfinite(attn_unified(q, wide[..., 1:129], v, "HND", dtype, False, True)).all()
+    k2 = k.expand(2, -1, -1, -1).contiguous()
+    k2[0, 1, 7, 5] = float("inf")
+    o = attn_unified(q, k2, v, "HND", dtype)
+    assert torch.isnan(o[0, 4:]).all() and torch.isfinite(o[0, :4]).all() and torch.isfinite(o[1]).all()
