@@ -101,3 +101,43 @@ def test_hybrid_layout_reads_selected_rows_from_pinned_host_memory():
     assert torch.equal(a, b)
     torch.cuda.synchronize()
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("k,d", [(32, 64), (96, 128), (1056, 128)])
+@pytest.mark.parametrize("kind", ["distinct", "ties", "one_score", "negative"])
+def test_selection_at_the_crossing_score(k, d, kind):
+    """The set of clusters that covers the budget, compared exactly with the oracle: budgets of one token, of all of them
+    and beyond, on and beside a cluster's edge; scores that tie across the crossing, that are all the same, and empty
+    clusters.  Centroids and queries are small integers, so every score is exact in any order."""
+    from longcontext_sqattn_paddle_b200 import _lib as L
+    from longcontext_sqattn_paddle_b200.ops import _stream
+    g = torch.Generator().manual_seed(k + len(kind))
+    groups, heads = 3, 2
+    q = torch.randint(-4, 5, (groups, heads, d), generator=g).to(torch.bfloat16)
+    cent = torch.randint(-8, 9, (groups, k, d), generator=g).to(torch.bfloat16)
+    if kind == "ties":
+        cent = cent[:, torch.arange(k) % 5].contiguous()
+    elif kind == "one_score":
+        cent = cent[:, :1].expand(-1, k, -1).contiguous()
+    elif kind == "negative":
+        q, cent = q.abs() + 1, -cent.abs() - 1
+    size = torch.randint(0, 9, (groups, k), generator=g, dtype=torch.int32)
+    size[0, :3] = 0
+    width = int(size.max())
+    total = int(size.sum(1).max())
+    lists = torch.zeros(groups, k, width, dtype=torch.int32)
+    for gi in range(groups):
+        perm, at = torch.randperm(total, generator=g).to(torch.int32), 0
+        for c in range(k):
+            n = int(size[gi, c])
+            lists[gi, c, :n] = perm[at:at + n].sort().values
+            at += n
+    qm = _mean_query(q.reshape(groups * heads, d), groups)
+    dev = [t.cuda().contiguous() for t in (q, cent, size, lists)]
+    out = torch.empty(groups, total, dtype=torch.int32, device="cuda")
+    cnt = torch.empty(groups, dtype=torch.int32, device="cuda")
+    for budget in (1, 2, 17, int(size[0].sum()) // 2, int(size[0].sum()), total + 5):
+        L.check(L.lib.sqattn_retrieve_select(dev[0].data_ptr(), dev[1].data_ptr(), L.BF16, dev[2].data_ptr(), dev[3].data_ptr(), groups,
+                                             heads, k, d, width, total, budget, out.data_ptr(), cnt.data_ptr(), total, total, _stream()))
+        for gi, sel in enumerate(ko.select_clusters(qm, cent, size, lists, budget)):
+            assert cnt[gi].item() == len(sel) and torch.equal(out[gi, :len(sel)].cpu(), sel)
