@@ -19,6 +19,7 @@ constexpr int kBlockM = 128;  // query rows per CTA (tcgen05 M)
 constexpr int kBlockN = 64;   // keys per step (the reference BLOCK_N)
 constexpr int kMaxSegs = 12;
 constexpr float kLazyLog2 = 8.0f;  // O is rescaled only when a row's maximum has moved by more than 2^8
+constexpr float kFp8Lead = 8.0f;   // kernels with an FP8 P: how far the reference of P, l and O starts below the maximum
 
 // segment flags
 constexpr int kSegAct0 = 1;   // rows 0..63 of the CTA take part
@@ -188,7 +189,9 @@ __device__ __forceinline__ void poison_output(const PrefillParams& p, int bi, in
   }
 }
 
-template <int D, bool kDump, int KS_, int VS_, int kMinCtas>
+// kFp8: some segment rounds P through e4m3 (an instantiation of its own: the rounding's registers and selects cost the
+// plain kernel 0.5 %)
+template <int D, bool kDump, int KS_, int VS_, int kMinCtas, bool kFp8>
 __global__ void __launch_bounds__(192, kMinCtas)
 prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant__ CUtensorMap tm_q4,
                const __grid_constant__ CUtensorMap tm_k8, const __grid_constant__ CUtensorMap tm_k4,
@@ -434,6 +437,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
     }
     for (StepIter it(segs, nseg); ok && !it.done(); it.next(), ++i) {
       const int flags = it.flags();
+      const bool fp8 = kFp8 && (flags & kSegFp8);
       const uint32_t s_tmem = tmem + lane_addr + (i & 1) * kBlockN;
       if (warp == 2 && lane == 0) SQ_STAMP(i, 5);
       ok = __all_sync(0xffffffffu, mbar_wait(bar_s_full + 8 * (i & 1), (i >> 1) & 1, cta_abort, 121));
@@ -441,7 +445,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
       tc_fence_after();
       if (warp == 2 && lane == 0) SQ_STAMP(i, 6);
       uint32_t pk[32];
-      float alpha = 1.0f;
+      float alpha = 1.0f, to_base = 1.0f;
       if (flags & half_bit) {
         uint32_t r0[32], r1[32];
         tmem_ld32(s_tmem, r0);
@@ -472,13 +476,17 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
         // P, l and O are kept relative to `base`, which follows the running maximum only when it has moved by
         // more than kLazyLog2 (so P <= 2^kLazyLog2): O then needs its rescale (a wait for the previous P V plus a
         // TMEM round trip) a few times per row instead of whenever the maximum moves.  Steps whose P is rounded
-        // through e4m3 keep base == running maximum, i.e. p <= 1 as the rounding rule expects.
-        const float thr = (flags & kSegFp8) ? 0.0f : kLazyLog2;
-        if (m_new > base + thr) {
-          alpha = ex2_approx(base - m_new);
-          base = m_new;
+        // through e4m3 round p = 2^(s - running maximum), as the rule says, and bring the rounded value to `base` with
+        // the factor 2^(m - base) in the multiplication that takes the 448 off again: still one rounding to f16.  There
+        // base stays kFp8Lead below the maximum it was set to, which keeps the smallest e4m3 values among f16's normal
+        // numbers (P <= 2^15).
+        if (m_new > base + (kFp8 ? kLazyLog2 + kFp8Lead - 1.0f : kLazyLog2)) {
+          const float to = kFp8 ? m_new - kFp8Lead : m_new;
+          alpha = ex2_approx(base - to);
+          base = to;
         }
-        const uint64_t m2 = f32x2_pack(base, base);
+        const float p_ref = fp8 ? m_new : base;
+        const uint64_t m2 = f32x2_pack(p_ref, p_ref);
         uint64_t sa = f32x2_pack(0.0f, 0.0f), sb = sa;
 #pragma unroll
         for (int c = 0; c < 64; c += 4) {
@@ -492,13 +500,17 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
         float s0, s1, s2, s3;
         f32x2_unpack(sa, s0, s1);
         f32x2_unpack(sb, s2, s3);
-        const float sum = (s0 + s1) + (s2 + s3);
+        float sum = (s0 + s1) + (s2 + s3);
+        if (fp8) { to_base = ex2_approx(m_new - base); sum *= to_base; }
         l_i = l_i * alpha + sum;
         if (warp == 2 && lane == 0) SQ_STAMP(i, 9);
         m_i = m_new;
-        if (flags & kSegFp8) {
+        if (fp8) {
+          const float f = to_base * (1.0f / 448.0f);
+          const __half fh = __float2half_rn(f), fl = __float2half_rn(f - __half2float(fh));
+          const __half2 hi = __half2half2(fh), lo = __half2half2(fl);
 #pragma unroll
-          for (int c = 0; c < 32; ++c) pk[c] = p_fp8_round_f16x2(x[2 * c], x[2 * c + 1]);
+          for (int c = 0; c < 32; ++c) pk[c] = p_fp8_times(x[2 * c], x[2 * c + 1], hi, lo);
         } else {
 #pragma unroll
           for (int c = 0; c < 32; ++c) pk[c] = pack_f16x2(x[2 * c], x[2 * c + 1]);
@@ -512,7 +524,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
         for (int c = 0; c < 32; ++c) {
           const __half2 h = *reinterpret_cast<const __half2*>(&pk[c]);
           float* dst = p.dump_p + (static_cast<size_t>(i) * kBlockM + row_in_tile) * 64 + 2 * c;
-          dst[0] = __low2float(h); dst[1] = __high2float(h);
+          dst[0] = __low2float(h) / to_base; dst[1] = __high2float(h) / to_base;   // relative to the step's maximum
         }
       }
       tmem_st32(s_tmem, pk);

@@ -199,18 +199,16 @@ int launch_prefill(const sqattn_prefill_args* a, const PrefillPlan& pl, cudaStre
   }
   const long long grid = static_cast<long long>(p.nblk) * Hq * B;
   if (grid > 0x7fffffffll) return fail(SQATTN_ERR_UNSUPPORTED, "grid too large");
-#define SQ_LAUNCH_PREFILL(KS, VS, MINB)                                                                                 \
+#define SQ_LAUNCH_PREFILL(DUMP, FP8)                                                                                     \
   do {                                                                                                                   \
-    using L = PrefillSmem<D, KS, VS>;                                                                                    \
-    if (dump || dump_t || dump_p) {                                                                                                \
-      SQ_CUDA(cudaFuncSetAttribute(prefill_kernel<D, true, KS, VS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynBytes)); \
-      prefill_kernel<D, true, KS, VS, MINB><<<static_cast<unsigned>(grid), 192, L::kDynBytes, stream>>>(tq8, tq4, tk8, tk4, tv, p);    \
-    } else {                                                                                                             \
-      SQ_CUDA(cudaFuncSetAttribute(prefill_kernel<D, false, KS, VS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynBytes)); \
-      prefill_kernel<D, false, KS, VS, MINB><<<static_cast<unsigned>(grid), 192, L::kDynBytes, stream>>>(tq8, tq4, tk8, tk4, tv, p);   \
-    }                                                                                                                    \
+    using L = PrefillSmem<D, 2, 3>;   /* two K stages (tied to the two S buffers), three V stages, two CTAs per SM */    \
+    auto kernel = prefill_kernel<D, DUMP, 2, 3, 2, FP8>;                                                                 \
+    SQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynBytes));                    \
+    kernel<<<static_cast<unsigned>(grid), 192, L::kDynBytes, stream>>>(tq8, tq4, tk8, tk4, tv, p);                       \
   } while (0)
-  SQ_LAUNCH_PREFILL(2, 3, 2);  // two K stages (tied to the two S buffers), three V stages, two CTAs per SM
+  if (dump || dump_t || dump_p) SQ_LAUNCH_PREFILL(true, true);
+  else if (a->p_fp8_mode) SQ_LAUNCH_PREFILL(false, true);
+  else SQ_LAUNCH_PREFILL(false, false);
 #undef SQ_LAUNCH_PREFILL
   SQ_CUDA(cudaGetLastError());
   return SQATTN_OK;
