@@ -9,7 +9,9 @@
 // While the epilogue warps of one token tile scan their 256 scores, the tensor core computes the other tile's, so
 // the two never wait for each other as long as a scan (about 3 instructions per score) is shorter than a tile's
 // 1024 tensor-pipe clocks.  Every centroid tile staged in shared memory is used by both token tiles, which halves
-// the L2 traffic per flop.
+// the L2 traffic per flop.  A CTA (one per SM) walks several 256-token items: with one item per CTA the start-up of
+// each (tensor memory, barriers, the first tiles) lay open: 268 us an assignment of 8 x 65536 keys to 1024 centroids, 220
+// now.  The scan's minima and maxima run at half rate, 107 us of it if nothing else stood in the way.
 //
 // Exactness: the fp32 tensor-core score is not the exact inner product, so a token whose best and second-best
 // scores are closer than a bound on that error is put on a list and re-scored in fp64 by kmeans_recheck_list_kernel
@@ -26,8 +28,9 @@ constexpr int kKtTokens = 256;    // tokens per CTA (two M = 128 tiles)
 constexpr int kKtCent = 256;      // centroids per MMA group (N)
 constexpr int kKtStages = 2;
 // |tensor-core fp32 sum - exact| is bounded by (terms * 2^-22) * sum|terms| <= 2^-15 |k||x| for 128 terms; the two
-// scores that are compared each carry it, and the factor of two on top covers an accumulator that truncates
-constexpr float kKtTol = 1.25e-4f;
+// scores that are compared each carry it, and the factor of two on top covers an accumulator that truncates.  The five
+// low bits that the epilogue spends on a score's column add 2^-18 |k||x| each.
+constexpr float kKtTol = 1.3e-4f;
 
 struct KmeansTcParams {
   const uint8_t* data;      // [G, T, D] for the token norms
@@ -36,7 +39,7 @@ struct KmeansTcParams {
   int* flagged_count;       // number of entries (may exceed cap: the overflow is re-scored by a full sweep)
   int flagged_cap;
   const float* max_cnorm2;  // [G] largest squared centroid norm of the group
-  int num_tokens, num_centroids, bf16;
+  int groups, num_tokens, num_centroids, bf16;
 };
 
 template <int D>
@@ -46,8 +49,8 @@ struct KmeansTcSmem {
   static constexpr int kAOff = 0;
   static constexpr int kBOff = 2 * kABytes;
   static constexpr int kBarOff = kBOff + kKtStages * kBBytes;
-  // a_full, b_full[2], s_full[2], s_empty[2]
-  static constexpr int kMiscOff = kBarOff + 8 * 7;
+  // a_full, b_full[2], s_full[2], s_empty[2], a_empty
+  static constexpr int kMiscOff = kBarOff + 8 * 8;
   static constexpr int kTotal = kMiscOff + 16;
 };
 
@@ -86,20 +89,25 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   const uint32_t sbase = smem_u32(smem);
-  const int g = blockIdx.y, t0 = blockIdx.x * kKtTokens;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto mark_all_for_recheck = [&]() {   // this CTA cannot deliver: every token of it goes through the exact path
-    for (int r = threadIdx.x; r < kKtTokens; r += blockDim.x)
-      if (t0 + r < p.num_tokens) p.idx[static_cast<long long>(g) * p.num_tokens + t0 + r] = -1;
-    if (threadIdx.x == 0) atomicAdd(p.flagged_count, p.flagged_cap + 1);   // forces the full sweep
+  // work items: (group, 256 tokens), group by group so that the CTAs that run together share centroids in L2
+  const int per_group = (p.num_tokens + kKtTokens - 1) / kKtTokens;
+  const long long items = static_cast<long long>(p.groups) * per_group;
+  auto mark_for_recheck = [&](long long from) {   // this CTA's items from `from` on go through the exact path
+    for (long long it = from; it < items; it += gridDim.x) {
+      const int g = static_cast<int>(it / per_group), t0 = static_cast<int>(it % per_group) * kKtTokens;
+      for (int r = threadIdx.x; r < kKtTokens; r += blockDim.x)
+        if (t0 + r < p.num_tokens) p.idx[static_cast<long long>(g) * p.num_tokens + t0 + r] = -1;
+    }
+    if (threadIdx.x == 0) atomicMax(p.flagged_count, p.flagged_cap + 1);   // forces the full sweep
   };
   if ((sbase & 1023u) || device_failed()) {
     if ((sbase & 1023u) && threadIdx.x == 0) record_failure(400);
-    mark_all_for_recheck();
+    mark_for_recheck(blockIdx.x);
     return;
   }
   const uint32_t a_s = sbase + L::kAOff, b_s = sbase + L::kBOff, bars = sbase + L::kBarOff;
-  const uint32_t bar_a_full = bars, bar_b_full = bars + 8, bar_s_full = bars + 24, bar_s_empty = bars + 40;
+  const uint32_t bar_a_full = bars, bar_b_full = bars + 8, bar_s_full = bars + 24, bar_s_empty = bars + 40, bar_a_empty = bars + 56;
   volatile uint32_t* tmem_base_s = reinterpret_cast<volatile uint32_t*>(smem + L::kMiscOff);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(smem + L::kMiscOff + 4);
   const int ntiles = (p.num_centroids + kKtCent - 1) / kKtCent;
@@ -109,6 +117,7 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
     mbar_init(bar_a_full, 1);
     for (int i = 0; i < kKtStages; ++i) mbar_init(bar_b_full + 8 * i, 1);
     for (int a = 0; a < 2; ++a) { mbar_init(bar_s_full + 8 * a, 1); mbar_init(bar_s_empty + 8 * a, 128); }
+    mbar_init(bar_a_empty, 256);
     fence_barrier_init();
     fence_proxy_async();
   }
@@ -121,26 +130,36 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
   tc_fence_after();
   const uint32_t tmem = *tmem_base_s;
 
+  // The barriers' phases run on over the items: `step` counts centroid tiles, `n` items.
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       tma_prefetch_desc(&tm_data); tma_prefetch_desc(&tm_cent);
-      mbar_expect_tx(bar_a_full, 2 * L::kABytes);
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int h = 0; h < D / 64; ++h)
-          tma_load_4d(a_s + a * L::kABytes + h * (128 * 128), &tm_data, bar_a_full, h * 64, t0 + a * 128, g, 0);
       bool ok = true;
-      for (int j = 0; ok && j < ntiles; ++j) {
-        const int st = j & 1;
-        // stage st was last read by the MMAs of tile j-2, token tile 1: their completion is s_full[1], phase j-2
-        if (j >= 2) ok = mbar_wait(bar_s_full + 8, (j - 2) & 1, cta_abort, 401);
-        if (!ok) break;
-        mbar_expect_tx(bar_b_full + 8 * st, L::kBBytes);
+      uint32_t step = 0, n = 0;
+      for (long long it = blockIdx.x; ok && it < items; it += gridDim.x, ++n) {
+        const int g = static_cast<int>(it / per_group), t0 = static_cast<int>(it % per_group) * kKtTokens;
+        for (int j = 0; ok && j < ntiles; ++j, ++step) {
+          const int st = step & 1;
+          // stage st was last read by the MMAs of step - 2, token tile 1: their completion is s_full[1], phase step - 2
+          if (step >= 2) ok = mbar_wait(bar_s_full + 8, (step - 2) & 1, cta_abort, 401);
+          if (!ok) break;
+          mbar_expect_tx(bar_b_full + 8 * st, L::kBBytes);
 #pragma unroll
-        for (int h = 0; h < D / 64; ++h)
-          tma_load_4d(b_s + st * L::kBBytes + h * (kKtCent * 128), &tm_cent, bar_b_full + 8 * st, h * 64, j * kKtCent, g, 0);
+          for (int h = 0; h < D / 64; ++h)
+            tma_load_4d(b_s + st * L::kBBytes + h * (kKtCent * 128), &tm_cent, bar_b_full + 8 * st, h * 64, j * kKtCent, g, 0);
+          if (j == 0) {
+            // the token tiles were last read by the MMAs of the previous step and by the epilogue (their norms)
+            if (n >= 1) ok = mbar_wait(bar_s_full + 8, (step - 1) & 1, cta_abort, 402) && mbar_wait(bar_a_empty, (n - 1) & 1, cta_abort, 403);
+            if (!ok) break;
+            mbar_expect_tx(bar_a_full, 2 * L::kABytes);
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+              for (int h = 0; h < D / 64; ++h)
+                tma_load_4d(a_s + a * L::kABytes + h * (128 * 128), &tm_data, bar_a_full, h * 64, t0 + a * 128, g, 0);
+          }
+        }
       }
     }
   } else if (warp == 1) {
@@ -148,24 +167,28 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
     {  // converged warp, one elected lane issues (operands stay warp-uniform values)
       const uint32_t fmt = p.bf16 ? 1u : 0u;
       const uint32_t idesc = make_idesc(fmt, fmt, 0, 0, 128, kKtCent);
-      bool ok = mbar_wait_warp(bar_a_full, 0, cta_abort, 411);
-      for (int j = 0; ok && j < ntiles; ++j) {
-        const int st = j & 1;
-        ok = mbar_wait_warp(bar_b_full + 8 * st, (j >> 1) & 1, cta_abort, 412);
-        if (!ok) break;
-        const uint64_t b_desc = smem_desc_sw128(b_s + st * L::kBBytes, 16, 1024);
-        for (int a = 0; ok && a < 2; ++a) {
-          if (j >= 1) ok = mbar_wait_warp(bar_s_empty + 8 * a, (j - 1) & 1, cta_abort, 413);
+      bool ok = true;
+      uint32_t step = 0, n = 0;
+      for (long long it = blockIdx.x; ok && it < items; it += gridDim.x, ++n) {
+        ok = mbar_wait_warp(bar_a_full, n & 1, cta_abort, 411);
+        for (int j = 0; ok && j < ntiles; ++j, ++step) {
+          const int st = step & 1;
+          ok = mbar_wait_warp(bar_b_full + 8 * st, (step >> 1) & 1, cta_abort, 412);
           if (!ok) break;
-          tc_fence_after();
-          const uint64_t a_desc = smem_desc_sw128(a_s + a * L::kABytes, 16, 1024);
+          const uint64_t b_desc = smem_desc_sw128(b_s + st * L::kBBytes, 16, 1024);
+          for (int a = 0; ok && a < 2; ++a) {
+            if (step >= 1) ok = mbar_wait_warp(bar_s_empty + 8 * a, (step - 1) & 1, cta_abort, 413);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t a_desc = smem_desc_sw128(a_s + a * L::kABytes, 16, 1024);
 #pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) {
-            const uint32_t off_a = (kk >> 2) * (128 * 128) + (kk & 3) * 32;
-            const uint32_t off_b = (kk >> 2) * (kKtCent * 128) + (kk & 3) * 32;
-            mma_ss_elect(tmem + a * kKtCent, a_desc + (off_a >> 4), b_desc + (off_b >> 4), idesc, kk > 0);
+            for (int kk = 0; kk < D / 16; ++kk) {
+              const uint32_t off_a = (kk >> 2) * (128 * 128) + (kk & 3) * 32;
+              const uint32_t off_b = (kk >> 2) * (kKtCent * 128) + (kk & 3) * 32;
+              mma_ss_elect(tmem + a * kKtCent, a_desc + (off_a >> 4), b_desc + (off_b >> 4), idesc, kk > 0);
+            }
+            tc_commit_elect(bar_s_full + 8 * a);
           }
-          tc_commit_elect(bar_s_full + 8 * a);
         }
       }
     }
@@ -174,75 +197,77 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
     const int a = (warp - 2) >> 2;              // token tile of this warp
     const int quarter = warp & 3;               // TMEM lanes this warp may touch: 32 * (warp % 4) ..
     const int row = quarter * 32 + lane;
-    const int tok = t0 + a * 128 + row;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    // |k|^2 of this thread's token, from global memory (the tile has just been loaded: an L2 hit)
-    float nrm2 = 0.f;
-    if (tok < p.num_tokens) {
-      const uint4* kr = reinterpret_cast<const uint4*>(p.data + (static_cast<long long>(g) * p.num_tokens + tok) * D * 2);
-      uint4 raw[D / 8];
-#pragma unroll
-      for (int ch = 0; ch < D / 8; ++ch) raw[ch] = kr[ch];          // all loads in flight before the first use
+    uint32_t keep = ~31u;                       // a score's low five bits make room for its column in the chunk
+    asm volatile("" : "+r"(keep));              // in a register: one three-input logic operation per score
+    bool ok = true;
+    uint32_t step = 0, n = 0;
+    for (long long it = blockIdx.x; it < items; it += gridDim.x, ++n) {
+      const int g = static_cast<int>(it / per_group), tok = static_cast<int>(it % per_group) * kKtTokens + a * 128 + row;
+      // |k|^2 of this thread's token, from the staged tile (16-byte chunk c of a row sits at c ^ (row & 7))
+      ok = mbar_wait_warp(bar_a_full, n & 1, cta_abort, 420);
+      if (!ok) break;
+      float nrm2 = 0.f;
+      const uint8_t* arow = smem + L::kAOff + a * L::kABytes + row * 128;
 #pragma unroll
       for (int ch = 0; ch < D / 8; ++ch) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(arow + (ch >> 3) * (128 * 128) + (((ch & 7) ^ (row & 7)) << 4));
         float f[8];
-        if (p.bf16) unpack8<true>(raw[ch], f); else unpack8<false>(raw[ch], f);
+        if (p.bf16) unpack8<true>(raw, f); else unpack8<false>(raw, f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) nrm2 += f[i] * f[i];
       }
-    }
-    float best = -INFINITY, second = -INFINITY;
-    int best_idx = 0;
-    bool ok = true;
-    for (int j = 0; ok && j < ntiles; ++j) {
-      ok = __all_sync(0xffffffffu, mbar_wait(bar_s_full + 8 * a, j & 1, cta_abort, 421));
-      if (!ok) break;
-      tc_fence_after();
-      const uint32_t s_tmem = tmem + lane_addr + a * kKtCent;
-      // num_centroids is a multiple of 32: a 32-column chunk is whole or absent
-      const int nch = min(kKtCent / 32, (p.num_centroids - j * kKtCent) / 32);
-      auto scan = [&](const uint32_t (&r)[32], int c0) {
-        const float before = best;
+      mbar_arrive(bar_a_empty);
+      float best = -INFINITY, second = -INFINITY;
+      int best_chunk = 0;
+      for (int j = 0; ok && j < ntiles; ++j, ++step) {
+        ok = mbar_wait_warp(bar_s_full + 8 * a, step & 1, cta_abort, 421);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t s_tmem = tmem + lane_addr + a * kKtCent;
+        // num_centroids is a multiple of 32: a 32-column chunk is whole or absent
+        const int nch = min(kKtCent / 32, (p.num_centroids - j * kKtCent) / 32);
+        // The column rides in the score's low bits, so the running maximum carries it along: two scores that differ by
+        // less than that are re-scored anyway.  Two at a time: the larger against the best, the rest against the second.
+        auto scan = [&](const uint32_t (&r)[32], int chunk) {
+          const float before = best;
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const float v = __uint_as_float(r[c]);
-          second = fmaxf(second, fminf(best, v));
-          best = fmaxf(best, v);
-        }
-        if (best > before) {                     // a new maximum inside this chunk: its first occurrence
-          int first = 31;
-#pragma unroll
-          for (int c = 31; c >= 0; --c)
-            if (__uint_as_float(r[c]) == best) first = c;
-          best_idx = c0 + first;
-        }
-      };
-      // two register buffers: the load of the next chunk is in flight while this one is scanned
-      uint32_t r0[32], r1[32];
-      tmem_ld32(s_tmem, r0);
+          for (int c = 0; c < 32; c += 2) {
+            const float v0 = __uint_as_float((r[c] & keep) | c), v1 = __uint_as_float((r[c + 1] & keep) | (c + 1));
+            const float hi = fmaxf(v0, v1), lo = fminf(v0, v1);
+            second = max3(second, lo, fminf(best, hi));
+            best = fmaxf(best, hi);
+          }
+          if (best > before) best_chunk = chunk;
+        };
+        // two register buffers: the load of the next chunk is in flight while this one is scanned
+        uint32_t r0[32], r1[32];
+        tmem_ld32(s_tmem, r0);
 #pragma unroll 1
-      for (int ch = 0; ch < nch; ch += 2) {
-        tmem_wait_ld();
-        if (ch + 1 < nch) tmem_ld32(s_tmem + (ch + 1) * 32, r1);
-        scan(r0, j * kKtCent + ch * 32);
-        if (ch + 1 < nch) {
+        for (int ch = 0; ch < nch; ch += 2) {
           tmem_wait_ld();
-          if (ch + 2 < nch) tmem_ld32(s_tmem + (ch + 2) * 32, r0);
-          scan(r1, j * kKtCent + (ch + 1) * 32);
+          if (ch + 1 < nch) tmem_ld32(s_tmem + (ch + 1) * 32, r1);
+          scan(r0, j * (kKtCent / 32) + ch);
+          if (ch + 1 < nch) {
+            tmem_wait_ld();
+            if (ch + 2 < nch) tmem_ld32(s_tmem + (ch + 2) * 32, r0);
+            scan(r1, j * (kKtCent / 32) + ch + 1);
+          }
         }
+        tc_fence_before();
+        mbar_arrive(bar_s_empty + 8 * a);
       }
-      tc_fence_before();
-      mbar_arrive(bar_s_empty + 8 * a);
-    }
-    ok = __all_sync(0xffffffffu, ok);
-    if (tok < p.num_tokens) {
-      const long long at = static_cast<long long>(g) * p.num_tokens + tok;
-      const float tol = kKtTol * sqrtf(nrm2) * sqrtf(p.max_cnorm2[g]);
-      const bool sure = ok && (best - second) > tol;
-      p.idx[at] = sure ? best_idx : (-1 - best_idx);
-      if (!sure) {
-        const int slot = atomicAdd(p.flagged_count, 1);
-        if (slot < p.flagged_cap) p.flagged[slot] = static_cast<int>(at);
+      if (!ok) break;
+      if (tok < p.num_tokens) {
+        const long long at = static_cast<long long>(g) * p.num_tokens + tok;
+        const int best_idx = best_chunk * 32 + static_cast<int>(__float_as_uint(best) & 31u);
+        const float tol = kKtTol * sqrtf(nrm2) * sqrtf(p.max_cnorm2[g]);
+        const bool sure = (best - second) > fmaxf(tol, 2e-38f);   // the columns of scores without a normal exponent are no order
+        p.idx[at] = sure ? best_idx : (-1 - best_idx);
+        if (!sure) {
+          const int slot = atomicAdd(p.flagged_count, 1);
+          if (slot < p.flagged_cap) p.flagged[slot] = static_cast<int>(at);
+        }
       }
     }
   }
@@ -253,6 +278,7 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
     while (globaltimer_ns() - t_wait < 200000ull) __nanosleep(1000);
   }
   __syncthreads();
+  if (*cta_abort) mark_for_recheck(blockIdx.x);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, kTmemCols);

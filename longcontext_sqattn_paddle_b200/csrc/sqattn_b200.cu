@@ -471,11 +471,12 @@ int km_launch_assign(const void* data, const void* centroids, int32_t dtype, int
   if ((rc = make_tmap_bhnd(&tc, centroids, dtype, sc * groups, sc, D, 1, groups, num_centroids, D, kKtCent, "kmeans centroids"))) return rc;
   KmeansTcParams p;
   p.data = static_cast<const uint8_t*>(data); p.idx = idx; p.flagged = w.flagged; p.flagged_count = w.flagged_count;
-  p.flagged_cap = w.flagged_cap; p.max_cnorm2 = w.max_cnorm2; p.num_tokens = num_tokens; p.num_centroids = num_centroids;
+  p.flagged_cap = w.flagged_cap; p.max_cnorm2 = w.max_cnorm2; p.groups = groups; p.num_tokens = num_tokens; p.num_centroids = num_centroids;
   p.bf16 = dtype == SQATTN_BF16;
   using L = KmeansTcSmem<D>;
   SQ_CUDA(cudaFuncSetAttribute(kmeans_assign_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-  const dim3 grid((num_tokens + kKtTokens - 1) / kKtTokens, groups);
+  const long long items = static_cast<long long>(groups) * ((num_tokens + kKtTokens - 1) / kKtTokens);
+  const unsigned grid = static_cast<unsigned>(items < 148 ? items : 148);   // persistent: one CTA per SM
   kmeans_assign_tc_kernel<D><<<grid, 320, L::kTotal, stream>>>(td, tc, p);
   SQ_CUDA(cudaGetLastError());
   return SQATTN_OK;
