@@ -495,7 +495,7 @@ int launch_window_hist_tc(const WindowHistParams& p, int dtype, cudaStream_t str
   if (smem < 116 * 1024) smem = 116 * 1024;   // one CTA per SM: each one allocates all of the tensor memory
   SQ_CUDA(cudaFuncSetAttribute(window_hist_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   const unsigned grid = static_cast<unsigned>((p.n + kWtRows - 1) / kWtRows) * p.hq;
-  window_hist_tc_kernel<D><<<grid, 320, smem, stream>>>(tq, tk, p, dtype == SQATTN_BF16);
+  window_hist_tc_kernel<D><<<grid, kWtThreads, smem, stream>>>(tq, tk, p, dtype == SQATTN_BF16);
   SQ_CUDA(cudaGetLastError());
   return SQATTN_OK;
 }
