@@ -250,11 +250,17 @@ struct DecodePlan {
   int lens[kDecMaxBatch];
 };
 
-// Length-aware scheduler: every work item covers `chunk` keys of one sequence; chunk is chosen so that all
-// sequences together give about ONE CTA per SM, never less than 256 keys per item.  Measured on B200 (1M keys,
-// 28/4 heads): one CTA per SM keeps 96 KB of loads in flight per SM, which already saturates HBM (6.6 TB/s), and
+// Length-aware scheduler: every work item covers `chunk` keys of one sequence, never less than 256.
+// One sequence: about ONE CTA per SM.  One keeps 96 KB of loads in flight, which already saturates HBM (6.6 TB/s), and
 // every further split only adds partial rows for the merge to read: 148 / 296 / 596 CTAs gave 162.7 / 165 / 178
-// microseconds per 1 GB layer shard and 4.3 / 7 / 16 microseconds of merge.
+// microseconds per 1 GB layer shard and 4.3 / 7 / 16 microseconds of merge (1M keys, 28/4 heads).
+// Several sequences: their ends leave items of any size, and a few CTAs more than SMs put two whole ones on some of them.
+// The smallest chunk that keeps the launch within one and a half CTAs per SM (two for more than eight sequences, which
+// leave more ends) lets the short items and the second halves fill up the memory system instead.  In a graph, before and
+// after: 8 sequences of 2000..65536 keys, 32/8 heads 122 and 112 us, 28/4 heads 69.6 and 62.4; 5 of 10000..40000 87 and
+// 79; 3 of 20000 52 and 48.5; beyond two CTAs per SM a second wave costs more than it evens out (121, 77, 96, 60).
+// Keys through an index list: two per SM as well, since the warps' own chain per tile bounds the kernel there (64 lists
+// of 4096 keys, FP8 P: 51 and 36 us; 56: 43 and 30; 16: 20 and 17).
 int plan_decode(const sqattn_decode_args* a, DecodePlan* pl) {
   if (!a) return fail(SQATTN_ERR_INVALID_ARG, "args is null");
   if (a->head_dim != 64 && a->head_dim != 128) return fail(SQATTN_ERR_UNSUPPORTED, "head_dim %d: only 64 and 128", a->head_dim);
@@ -291,6 +297,23 @@ int plan_decode(const sqattn_decode_args* a, DecodePlan* pl) {
   } else {
     const long long target = (148ll + a->num_kv_heads - 1) / a->num_kv_heads;  // items per KV head
     chunk = static_cast<int>((total_tiles + target - 1) / target) * kDecTile;
+    const long long most = (a->gather || a->batch > 8 ? 296ll : 222ll) / a->num_kv_heads;
+    if ((a->batch > 1 || a->gather) && most > a->batch && total_tiles > 0) {
+      auto items_of = [&](long long c) {
+        long long n = 0;
+        for (int b = 0; b < a->batch; ++b) n += (pl->lens[b] + c - 1) / c;
+        return n;
+      };
+      // the smallest chunk (in tiles) with at most `most` items: the count falls as the chunk grows
+      long long lo = (total_tiles + most - 1) / most, hi = chunk / kDecTile;
+      if (lo < 1) lo = 1;
+      while (items_of(hi * kDecTile) > most) hi *= 2;
+      while (lo < hi) {
+        const long long mid = (lo + hi) / 2;
+        if (items_of(mid * kDecTile) > most) lo = mid + 1; else hi = mid;
+      }
+      chunk = static_cast<int>(lo) * kDecTile;
+    }
   }
   chunk = (chunk + kDecTile - 1) / kDecTile * kDecTile;
   if (chunk < 256) chunk = 256;
