@@ -4,6 +4,7 @@ include/sqattn_b200.h.  No arithmetic happens on the Python side."""
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from typing import Optional, Sequence
 
 import torch
@@ -20,7 +21,8 @@ def _dt(dtype: torch.dtype) -> int:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current device's current stream, without building a Stream object (a microsecond of every call)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _require_cuda(*ts):
@@ -29,14 +31,47 @@ def _require_cuda(*ts):
             raise RuntimeError("sqattn_b200 runs on CUDA tensors only (there is no CPU path)")
 
 
-def _view(t: torch.Tensor, layout: str) -> L.Tensor:
-    """Logical [B,H,N,D] view of a 4-D tensor stored HND or NHD."""
-    assert t.dim() == 4 and t.stride(-1) == 1, "Last dim of qkv must be contiguous."
+def _desc(t: torch.Tensor, layout: str):
+    """(pointer, batch, head and token strides) of the logical [B,H,N,D] view of a 4-D tensor stored HND or NHD."""
+    st = t.stride()
+    assert len(st) == 4 and st[3] == 1, "Last dim of qkv must be contiguous."
     if layout == "HND":
-        return L.Tensor(t.data_ptr(), t.stride(0), t.stride(1), t.stride(2))
+        return t.data_ptr(), st[0], st[1], st[2]
     if layout == "NHD":
-        return L.Tensor(t.data_ptr(), t.stride(0), t.stride(2), t.stride(1))
+        return t.data_ptr(), st[0], st[2], st[1]
     raise ValueError(f"tensor_layout {layout} not supported")
+
+
+def _view(t: torch.Tensor, layout: str) -> L.Tensor:
+    return L.Tensor(*_desc(t, layout))
+
+
+_NO_TENSOR = (0, 0, 0, 0)
+_PREFILL_TENSORS = struct.Struct("25q")   # q_int8, k_int8, q_int4, k_int4, v, o of sqattn_prefill_args, and lse
+assert L.PrefillArgs.lse.offset == _PREFILL_TENSORS.size - 8
+# sqattn_decode_args in the header's order, filled in one call: setting its 45 fields one by one through ctypes took
+# about as long as the launches
+_DECODE_ARGS = struct.Struct("4q4q4q4qq5i4xq6iqQqqqqi4xq")
+assert _DECODE_ARGS.size == C.sizeof(L.DecodeArgs)
+
+
+def _decode_args(q, k, v, o, lse, batch, hq, hkv, d, kv_len, dtype, o_dtype, *, kv_lens=0, p_fp8=False, q_is_scaled=False, num_splits=0,
+                 reference_tail=False, partial_o=0, partial_lse=0, kv_lens_device=0, peer=0, head_dim_og=0, gather=0) -> L.DecodeArgs:
+    """q, k, v, o as _desc gives them; pointers as integers."""
+    return L.DecodeArgs.from_buffer(bytearray(_DECODE_ARGS.pack(
+        *q, *k, *v, *o, lse, batch, hq, hkv, d, kv_len, kv_lens, dtype, o_dtype, int(p_fp8), int(q_is_scaled), int(num_splits),
+        int(reference_tail), 0, 0, partial_o, partial_lse, kv_lens_device, peer, int(head_dim_og), gather)))
+
+
+def _run_decode(a: L.DecodeArgs, device, workspace_bytes, entry):
+    """Workspace and launch.  A rejected plan (0 bytes) goes on to the entry point, which reports why."""
+    need = workspace_bytes(C.byref(a))
+    if need:
+        ws = torch.empty(need, dtype=torch.uint8, device=device)   # the caching allocator's blocks are 512-byte aligned
+        a.workspace, a.workspace_bytes = ws.data_ptr(), need
+    L.check(entry(C.byref(a), _stream()))
+    if not need:
+        raise ValueError("sqattn_decode: invalid arguments")
 
 
 def _shape(t: torch.Tensor, layout: str):
@@ -73,7 +108,7 @@ def _workspace(nbytes: int, device) -> Optional[torch.Tensor]:
         return None
     ws = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
     off = (-ws.data_ptr()) % 1024
-    return ws[off:off + nbytes]
+    return ws[off:off + nbytes] if off else ws
 
 
 def prefill(q8, k8, q4, k4, v, *, mode: int, win8=None, win4=None, sink: int = 0, layout: str = "HND",
@@ -94,29 +129,29 @@ def prefill(q8, k8, q4, k4, v, *, mode: int, win8=None, win4=None, sink: int = 0
         out = torch.empty(q8.shape, dtype=out_dtype, device=q8.device)
         out_layout = layout
     lse = torch.empty(b, hq, n, dtype=torch.float32, device=q8.device) if return_lse else None
-    a = L.PrefillArgs()
-    a.q_int8, a.k_int8 = _view(q8, layout), _view(k8, kv_layout)
-    a.q_int4, a.k_int4 = _view(q4, layout), _view(k4, kv_layout)
-    a.v, a.o = _view(v, kv_layout), _view(out, out_layout)
+    qd, kd = _desc(q8, layout), _desc(k8, kv_layout)
+    buf = bytearray(C.sizeof(L.PrefillArgs))
+    _PREFILL_TENSORS.pack_into(buf, 0, *qd, *kd, *(qd if q4 is q8 else _desc(q4, layout)), *(kd if k4 is k8 else _desc(k4, kv_layout)),
+                               *_desc(v, kv_layout), *_desc(out, out_layout), 0 if lse is None else lse.data_ptr())
+    a = L.PrefillArgs.from_buffer(buf)
     a.q_row_offset, a.head_dim_og = int(q_row_offset), int(head_dim_og)
     a.q_split_rows, a.q_row_offset2 = int(q_split_rows), int(q_row_offset2)   # second row range of a shard, if any
     if q_fake_quant is not None:
         if q_fake_quant not in L.QTYPE:
             raise ValueError(f"Invalid quantization type: {q_fake_quant}")
         a.q_fake_quant, a.q_round_half_even = L.QTYPE[q_fake_quant] + 1, int(round_half_even)
-    a.lse = lse.data_ptr() if lse is not None else None
     a.batch, a.num_q_heads, a.num_kv_heads, a.qo_len, a.kv_len, a.head_dim = b, hq, hkv, n, kv_len, d
     a.qk_dtype, a.v_dtype, a.o_dtype = _dt(q8.dtype), _dt(v.dtype), _dt(out.dtype)
     a.mode, a.sink_size, a.p_fp8_mode, a.q_is_scaled = mode, int(sink), int(p_fp8_mode), int(q_is_scaled)
     keep = []
     if mode == L.MODE_RELATIVE_WINDOW:
-        r8 = (C.c_float * hq)(*[float(x) for x in win8])
-        r4 = (C.c_float * hq)(*[float(x) for x in win4])
+        r8 = (C.c_float * hq)(*map(float, win8))
+        r4 = (C.c_float * hq)(*map(float, win4))
         a.win8_ratios, a.win4_ratios = r8, r4
         keep += [r8, r4]
     elif mode == L.MODE_ABSOLUTE_WINDOW:
-        s8 = (C.c_int32 * hq)(*[int(x) for x in win8])
-        s4 = (C.c_int32 * hq)(*[int(x) for x in win4])
+        s8 = (C.c_int32 * hq)(*map(int, win8))
+        s4 = (C.c_int32 * hq)(*map(int, win4))
         a.win8_sizes, a.win4_sizes = s8, s4
         keep += [s8, s4]
     need = L.lib.sqattn_prefill_workspace_bytes(C.byref(a))
@@ -173,7 +208,7 @@ def prep_qkv(query, key, value, *, qk_qtype: str = "int", v_qtype: str = "int", 
         assert k_mean.dtype == torch.float32 and k_mean.is_contiguous() and k_mean.shape == (b, hkv, d)
         a.k_mean = k_mean.data_ptr()
     need = L.lib.sqattn_prep_workspace_bytes(C.byref(a))
-    ws = _workspace(need, dev)
+    ws = torch.empty(need, dtype=torch.uint8, device=dev)
     a.workspace, a.workspace_bytes = ws.data_ptr(), need
     L.check(L.lib.sqattn_prep_qkv(C.byref(a), _stream()))
     return q8, q4, k8, k4, v8
@@ -209,44 +244,30 @@ def decode(q, k, v, *, layout: str = "HND", out_dtype=torch.float16, return_lse:
     b, hq, one, d = _shape(q, layout)
     assert one == 1
     _, hkv, cap, _ = _shape(k, layout)
-    a = L.DecodeArgs()
-    a.q, a.k, a.v = _view(q, layout), _view(k, layout), _view(v, layout)
-    a.batch, a.num_q_heads, a.num_kv_heads, a.head_dim, a.head_dim_og = b, hq, hkv, d, int(head_dim_og)
-    a.kv_len = int(cap if kv_len is None else kv_len)
     lens = None
     if kv_lens is not None:
         lens = (C.c_int32 * b)(*[int(x) for x in kv_lens])
-        a.kv_lens = lens
-    a.dtype, a.p_fp8, a.q_is_scaled, a.num_splits = _dt(k.dtype), int(p_fp8), int(q_is_scaled), int(num_splits)
-    a.reference_tail = int(reference_tail)
     if kv_lens_device is not None:
         if kv_lens is not None:
             raise ValueError("kv_lens and kv_lens_device are exclusive: device lengths are planned for kv_len")
         assert kv_lens_device.is_cuda and kv_lens_device.dtype == torch.int32 and kv_lens_device.numel() == b
-        a.kv_lens_device = kv_lens_device.data_ptr()
     out = lse = po = pl = None
-    if peer is not None:
-        a.peer = C.addressof(peer)
-        a.o_dtype = L.F16
-    elif partial:
+    o_desc, o_dtype = _NO_TENSOR, L.F16
+    if peer is None and partial:
         po = torch.empty(b, hq, d, dtype=torch.float32, device=q.device)
         pl = torch.empty(b, hq, dtype=torch.float32, device=q.device)
-        a.partial_o, a.partial_lse = po.data_ptr(), pl.data_ptr()
-        a.o_dtype = L.F16
-    else:
+    elif peer is None:
         out = torch.empty(q.shape, dtype=out_dtype, device=q.device)
-        a.o = _view(out, layout)
-        a.o_dtype = _dt(out_dtype)
+        o_desc, o_dtype = _desc(out, layout), _dt(out_dtype)
         if return_lse:
             lse = torch.empty(b, hq, 1, dtype=torch.float32, device=q.device)
-            a.lse = lse.data_ptr()
-    need = L.lib.sqattn_decode_workspace_bytes(C.byref(a))
-    if need == 0:  # the plan was rejected: let the entry point report why
-        L.check(L.lib.sqattn_decode(C.byref(a), _stream()))
-        raise ValueError("sqattn_decode: invalid arguments")
-    ws = _workspace(need, q.device)
-    a.workspace, a.workspace_bytes = ws.data_ptr(), need
-    L.check(L.lib.sqattn_decode(C.byref(a), _stream()))
+    a = _decode_args(_desc(q, layout), _desc(k, layout), _desc(v, layout), o_desc, 0 if lse is None else lse.data_ptr(), b, hq, hkv, d,
+                     int(cap if kv_len is None else kv_len), _dt(k.dtype), o_dtype, kv_lens=0 if lens is None else C.addressof(lens),
+                     p_fp8=p_fp8, q_is_scaled=q_is_scaled, num_splits=num_splits, reference_tail=reference_tail,
+                     partial_o=0 if po is None else po.data_ptr(), partial_lse=0 if pl is None else pl.data_ptr(),
+                     kv_lens_device=0 if kv_lens_device is None else kv_lens_device.data_ptr(),
+                     peer=0 if peer is None else C.addressof(peer), head_dim_og=head_dim_og)
+    _run_decode(a, q.device, L.lib.sqattn_decode_workspace_bytes, L.lib.sqattn_decode)
     if peer is not None:
         return None
     if partial:
@@ -254,12 +275,10 @@ def decode(q, k, v, *, layout: str = "HND", out_dtype=torch.float16, return_lse:
     return (out, lse) if return_lse else out
 
 
-def tma_ready(t: torch.Tensor, layout: str) -> bool:
+def tma_ready(t: torch.Tensor) -> bool:
     """The kernels can read ``t`` where it lies: 16-byte aligned rows, no broadcast dimension."""
-    b, h, n, d = _shape(t, layout)
-    v = _view(t, layout) if t.stride(-1) == 1 else None
-    return v is not None and t.data_ptr() % 16 == 0 and all(
-        s % 8 == 0 and (s > 0 or ext == 1) for s, ext in ((v.stride_b, b), (v.stride_h, h), (v.stride_n, n)))
+    st = t.stride()
+    return st[3] == 1 and t.data_ptr() % 16 == 0 and all(s % 8 == 0 and (s > 0 or ext == 1) for s, ext in zip(st[:3], t.shape))
 
 
 def decode_centered(q, k, v, *, layout: str = "HND", out_dtype=torch.float16, return_lse: bool = False,
@@ -270,17 +289,11 @@ def decode_centered(q, k, v, *, layout: str = "HND", out_dtype=torch.float16, re
     b, hq, one, d = _shape(q, layout)
     assert one == 1
     _, hkv, cap, _ = _shape(k, layout)
-    a = L.DecodeArgs()
     out = torch.empty(q.shape, dtype=out_dtype, device=q.device)
     lse = torch.empty(b, hq, 1, dtype=torch.float32, device=q.device) if return_lse else None
-    a.q, a.k, a.v, a.o = _view(q, layout), _view(k, layout), _view(v, layout), _view(out, layout)
-    a.batch, a.num_q_heads, a.num_kv_heads, a.head_dim, a.head_dim_og = b, hq, hkv, d, int(head_dim_og)
-    a.kv_len, a.dtype, a.o_dtype, a.reference_tail = cap, _dt(k.dtype), _dt(out_dtype), int(reference_tail)
-    a.lse = lse.data_ptr() if return_lse else None
-    need = L.lib.sqattn_decode_centered_workspace_bytes(C.byref(a))
-    ws = _workspace(need, q.device)    # 0: the plan was rejected, the entry point reports why
-    a.workspace, a.workspace_bytes = (ws.data_ptr() if ws is not None else None), need
-    L.check(L.lib.sqattn_decode_centered(C.byref(a), _stream()))
+    a = _decode_args(_desc(q, layout), _desc(k, layout), _desc(v, layout), _desc(out, layout), lse.data_ptr() if return_lse else 0,
+                     b, hq, hkv, d, cap, _dt(k.dtype), _dt(out_dtype), reference_tail=reference_tail, head_dim_og=head_dim_og)
+    _run_decode(a, q.device, L.lib.sqattn_decode_centered_workspace_bytes, L.lib.sqattn_decode_centered)
     return (out, lse) if return_lse else out
 
 
@@ -298,23 +311,10 @@ def decode_gather(q, idx, counts, k_rows, v_rows, row_stride: int, kv_dtype, *, 
     assert k_rows.dtype == torch.int64 and v_rows.dtype == torch.int64 and k_rows.numel() == b * num_kv_heads == v_rows.numel()
     g = L.DecodeGather()
     g.idx, g.cap, g.k_rows, g.v_rows, g.row_stride = idx.data_ptr(), idx.shape[1], k_rows.data_ptr(), v_rows.data_ptr(), int(row_stride)
-    a = L.DecodeArgs()
-    a.q = _view(q, "HND")
-    a.batch, a.num_q_heads, a.num_kv_heads, a.head_dim = b, hq, num_kv_heads, d
-    a.kv_len = idx.shape[1]
-    a.dtype, a.p_fp8, a.q_is_scaled = _dt(kv_dtype), int(p_fp8), int(q_is_scaled)
-    a.kv_lens_device = counts.data_ptr()
-    a.gather = C.addressof(g)
     out = torch.empty(q.shape, dtype=out_dtype, device=q.device)
-    a.o = _view(out, "HND")
-    a.o_dtype = _dt(out_dtype)
-    need = L.lib.sqattn_decode_workspace_bytes(C.byref(a))
-    if need == 0:  # the plan was rejected: let the entry point report why
-        L.check(L.lib.sqattn_decode(C.byref(a), _stream()))
-        raise ValueError("sqattn_decode: invalid arguments")
-    ws = _workspace(need, q.device)
-    a.workspace, a.workspace_bytes = ws.data_ptr(), need
-    L.check(L.lib.sqattn_decode(C.byref(a), _stream()))
+    a = _decode_args(_desc(q, "HND"), _NO_TENSOR, _NO_TENSOR, _desc(out, "HND"), 0, b, hq, num_kv_heads, d, idx.shape[1], _dt(kv_dtype),
+                     _dt(out_dtype), p_fp8=p_fp8, q_is_scaled=q_is_scaled, kv_lens_device=counts.data_ptr(), gather=C.addressof(g))
+    _run_decode(a, q.device, L.lib.sqattn_decode_workspace_bytes, L.lib.sqattn_decode)
     return out
 
 

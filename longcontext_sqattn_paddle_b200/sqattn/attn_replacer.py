@@ -70,16 +70,16 @@ def mp_triton_wrapper(layer_idx, bit8_window_sizes=0, bit4_window_sizes=0, sink_
         out = torch.empty(b, n, hq * d, dtype=torch.bfloat16, device=query.device)
         o4 = out.view(b, n, hq, d)
 
-        def per_head(w, conv):
-            return [conv(w)] * hq if isinstance(w, (int, float)) else [conv(x) for x in w]
+        def per_head(w):
+            return [w] * hq if isinstance(w, (int, float)) else w
 
         if relative:
-            ops.prefill(q8, k8, q8, k8, v8, mode=L.MODE_RELATIVE_WINDOW, win8=per_head(bit8_window_sizes, float),
-                        win4=per_head(bit4_window_sizes, float), sink=sink_window_size, layout="HND",
+            ops.prefill(q8, k8, q8, k8, v8, mode=L.MODE_RELATIVE_WINDOW, win8=per_head(bit8_window_sizes),
+                        win4=per_head(bit4_window_sizes), sink=sink_window_size, layout="HND",
                         p_fp8_mode=fp8, q_is_scaled=True, out=o4, out_layout="NHD")
         else:
-            ops.prefill(q8, k8, q4, k4, v8, mode=L.MODE_ABSOLUTE_WINDOW, win8=per_head(bit8_window_sizes, int),
-                        win4=per_head(bit4_window_sizes, int), sink=sink_window_size, layout="HND",
+            ops.prefill(q8, k8, q4, k4, v8, mode=L.MODE_ABSOLUTE_WINDOW, win8=per_head(bit8_window_sizes),
+                        win4=per_head(bit4_window_sizes), sink=sink_window_size, layout="HND",
                         p_fp8_mode=fp8, q_is_scaled=True, out=o4, out_layout="NHD")
         return out
 

@@ -101,7 +101,7 @@ def attn_unified(q, k, v, tensor_layout="HND", output_dtype=torch.float16, retur
     seq_dim = 1 if tensor_layout == "NHD" else 2
     if (center_k and kv_lens is None and not is_P_fp8_quant and tensor_layout in ("HND", "NHD") and q.shape[seq_dim] == 1
             and q.dim() == k.dim() == 4 and q.shape[-1] in (64, 128) and q.dtype == k.dtype == v.dtype
-            and k.dtype in (torch.float16, torch.bfloat16) and k.is_cuda and k.numel() and ops.tma_ready(k, tensor_layout)):
+            and k.dtype in (torch.float16, torch.bfloat16) and k.is_cuda and k.numel() and ops.tma_ready(k)):
         return ops.decode_centered(q, k, v, layout=tensor_layout, out_dtype=output_dtype, return_lse=return_lse,
                                    reference_tail=True)
     if center_k:
