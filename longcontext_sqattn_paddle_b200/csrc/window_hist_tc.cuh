@@ -3,7 +3,7 @@
 //
 // What bounds it: one exponential per (query, key) pair.  The mma.sync kernel swept the keys twice (statistics, then
 // normalised weights), computed two exponentials and an IEEE division per pair and took 10.6 ms for 28 heads x 8192
-// tokens x 200 bins (this one 1.13 ms); the products of one sweep are 0.15 ms of the measured tensor rate, its exponentials 0.2 ms of the
+// tokens x 200 bins (this one 1.10 ms); the products of one sweep are 0.15 ms of the measured tensor rate, its exponentials 0.2 ms of the
 // special-function units.  Hence:
 //   * a thread owns one query row (a TMEM lane) and meets its keys in order, so its bins never increase: a bin is one
 //     run, kept as A0 = sum a and A1 = sum a * (j - ref) with a = 2^(score - base) NOT normalised, and stored once, in a
@@ -30,7 +30,6 @@ constexpr int kWtRows = 128, kWtKeys = 64, kWtParts = 4;
 constexpr int kWtThreads = 64 + kWtParts * 128;
 constexpr int kWtMaxBins = 248;       // nbins x 128 fp32 + Q tile + one K stage per part within 227 KB
 constexpr int kWtKeysPerBin = 1024;   // seq_len / nbins at most this (edge(): at most one distance near an edge)
-constexpr int kWtFastWidth = 9;       // bins at least this wide (keys): at most one edge among eight consecutive keys
 constexpr float kWtLazyLog2 = 60.0f;
 
 template <int D>
@@ -130,7 +129,10 @@ struct WindowRow {
   }
   __device__ __forceinline__ float shift() const { return base == -INFINITY ? 0.f : -(base * c2); }
 
-  // 32 keys from c0 on, all of them visible and behind the sink, bins at least kWtFastWidth wide
+  // 32 keys from c0 on, all of them visible and behind the sink, bins wider than kSub keys: at most one edge among kSub
+  // consecutive keys.  The lanes' edges lie all over the chunk, so every group of kSub keys splits its sums at the edge by
+  // predicate, and the lanes that have one there end their runs together.
+  template <int kSub>
   __device__ __forceinline__ void chunk32(const uint32_t (&r)[32], int c0) {
     float mx = max3(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]));
 #pragma unroll
@@ -138,27 +140,22 @@ struct WindowRow {
     look_at_max(fmaxf(mx, __uint_as_float(r[31])));
     if (cur < 0) begin(c0);
     const float sh = shift(), t0 = weight(c0);
+    float x[32];
 #pragma unroll
-    for (int s = 0; s < 32; s += 8) {
+    for (int c = 0; c < 32; ++c) x[c] = ex2_approx(__fmaf_rn(__uint_as_float(r[c]), c2, sh));
+#pragma unroll
+    for (int s = 0; s < 32; s += kSub) {
       const int nb = next - c0;
-      float x[8];
+      float v0 = 0.f, v1 = 0.f;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) x[e] = ex2_approx(__fmaf_rn(__uint_as_float(r[s + e]), c2, sh));
-      if (__any_sync(0xffffffffu, nb < s + 8)) {
-        float v0 = 0.f, v1 = 0.f;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          if (s + e < nb) { a0 += x[e]; a1 = __fmaf_rn(x[e], static_cast<float>(s + e), a1); }
-          else { v0 += x[e]; v1 = __fmaf_rn(x[e], static_cast<float>(s + e), v1); }
-        }
-        if (nb < s + 8) {
-          flush(t0);
-          a0 = v0; a1 = v1;
-          lower();
-        }
-      } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) { a0 += x[e]; a1 = __fmaf_rn(x[e], static_cast<float>(s + e), a1); }
+      for (int c = s; c < s + kSub; ++c) {
+        if (c < nb) { a0 += x[c]; a1 = __fmaf_rn(x[c], static_cast<float>(c), a1); }
+        else { v0 += x[c]; v1 = __fmaf_rn(x[c], static_cast<float>(c), v1); }
+      }
+      if (nb < s + kSub) {
+        flush(t0);
+        a0 = v0; a1 = v1;
+        lower();
       }
     }
     a1 = __fmaf_rn(-32.0f, a0, a1);
@@ -316,7 +313,8 @@ window_hist_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     w.hist = hist + row; w.aside = g ? aside_s + g * 128 + row : nullptr; w.slot = w.hist; w.tie = tie_s;
     w.base = -INFINITY; w.a0 = w.a1 = w.l = 0.f; w.cur = w.first = -1; w.next = 0x7fffffff;
     w.eq = w.er = 0;
-    const bool wide = i_first + 31 < p.n && i_first - p.sink >= kWtFastWidth * p.nbins;
+    // bins of 9 (17) keys and more: their edges are at least 8 (16) keys apart, rounded or not
+    const bool wide = i_first + 31 < p.n && i_first - p.sink >= 9 * p.nbins, very_wide = wide && i_first - p.sink >= 17 * p.nbins;
     bool ok = true;
     int ref = 0;                                                        // key that a1 is relative to
     const int tile0 = part_begin(g), tiles = part_begin(g + 1) - tile0;
@@ -333,7 +331,8 @@ window_hist_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           uint32_t r[32];
           tmem_ld32(s_tmem + c, r);
           tmem_wait_ld();
-          w.chunk32(r, j0 + c);
+          if (very_wide) w.chunk32<16>(r, j0 + c);
+          else w.chunk32<8>(r, j0 + c);
           c += 32;
         } else {
           uint32_t r[8];
