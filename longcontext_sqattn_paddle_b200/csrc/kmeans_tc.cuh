@@ -410,7 +410,7 @@ kmeans_recheck_list_kernel(const uint8_t* data, const uint8_t* cent, int* idx, c
     if (threadIdx.x == 0) {
       for (int w = 1; w < 8; ++w)
         if (best_s[w] > best || (best_s[w] == best && idx_s[w] < bi)) { best = best_s[w]; bi = idx_s[w]; }
-      idx[at] = bi;
+      idx[at] = bi < num_centroids ? bi : 0;   // no candidate at all: a NaN key
     }
   }
 }
@@ -589,7 +589,7 @@ constexpr int kSortClusters = 49152;
 __global__ void __launch_bounds__(32) kmeans_range_count_kernel(const int* idx, int* hist, int num_tokens, int num_centroids, int per_range,
                                                                 int c0, int nc) {
   extern __shared__ int cnt_s[];
-  const int g = blockIdx.y, r = blockIdx.x, lane = threadIdx.x;
+  const int g = blockIdx.x, r = blockIdx.y, lane = threadIdx.x;
   for (int c = lane; c < nc; c += 32) cnt_s[c] = 0;
   __syncwarp();
   const int t0 = r * per_range, t1 = min(num_tokens, t0 + per_range);
@@ -600,12 +600,12 @@ __global__ void __launch_bounds__(32) kmeans_range_count_kernel(const int* idx, 
     if (c >= 0 && c < nc) atomicAdd(cnt_s + c, 1);
   }
   __syncwarp();
-  int* hg = hist + (static_cast<long long>(g) * gridDim.x + r) * num_centroids + c0;
+  int* hg = hist + (static_cast<long long>(g) * gridDim.y + r) * num_centroids + c0;
   for (int c = lane; c < nc; c += 32) hg[c] = cnt_s[c];
 }
 // hist[g, r, c] <- members of c in the ranges before r;  cluster_size[g, c] = all of them.  A thread per cluster.
 __global__ void __launch_bounds__(256) kmeans_range_scan_kernel(int* hist, int* cluster_size, int ranges, int num_centroids) {
-  const int c = blockIdx.x * 256 + threadIdx.x, g = blockIdx.y;
+  const int c = blockIdx.y * 256 + threadIdx.x, g = blockIdx.x;
   if (c >= num_centroids) return;
   int* h = hist + static_cast<long long>(g) * ranges * num_centroids + c;
   int run = 0;
@@ -625,8 +625,8 @@ __global__ void __launch_bounds__(32) kmeans_range_emit_kernel(const int* idx, c
                                                                int num_centroids, int per_range, int max_cluster_size,
                                                                int c0, int nc) {
   extern __shared__ int next_s[];
-  const int g = blockIdx.y, r = blockIdx.x, lane = threadIdx.x;
-  const int* hg = hist + (static_cast<long long>(g) * gridDim.x + r) * num_centroids + c0;
+  const int g = blockIdx.x, r = blockIdx.y, lane = threadIdx.x;
+  const int* hg = hist + (static_cast<long long>(g) * gridDim.y + r) * num_centroids + c0;
   for (int c = lane; c < nc; c += 32) next_s[c] = hg[c];
   __syncwarp();
   const int t0 = r * per_range, t1 = min(num_tokens, t0 + per_range);

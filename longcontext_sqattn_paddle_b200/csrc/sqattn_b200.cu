@@ -853,14 +853,14 @@ int sqattn_kmeans_reverse_index(const int32_t* idx, int32_t groups, int32_t num_
   // a range is a multiple of 32 tokens, at least 256 of them
   int per_range = ((num_tokens + kSortRanges - 1) / kSortRanges + 31) / 32 * 32;
   if (per_range < 256) per_range = 256;
-  const dim3 ranges((num_tokens + per_range - 1) / per_range, groups);
+  const dim3 ranges(groups, (num_tokens + per_range - 1) / per_range);   // any number of groups
   const int smem = (num_centroids < kSortClusters ? num_centroids : kSortClusters) * static_cast<int>(sizeof(int));
   SQ_CUDA(cudaFuncSetAttribute(kmeans_range_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   SQ_CUDA(cudaFuncSetAttribute(kmeans_range_emit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   for (int c0 = 0; c0 < num_centroids; c0 += kSortClusters)
     kmeans_range_count_kernel<<<ranges, 32, smem, stream>>>(idx, w.range_hist, num_tokens, num_centroids, per_range, c0,
                                                             num_centroids - c0 < kSortClusters ? num_centroids - c0 : kSortClusters);
-  kmeans_range_scan_kernel<<<dim3((num_centroids + 255) / 256, groups), 256, 0, stream>>>(w.range_hist, cluster_size, ranges.x, num_centroids);
+  kmeans_range_scan_kernel<<<dim3(groups, (num_centroids + 255) / 256), 256, 0, stream>>>(w.range_hist, cluster_size, ranges.y, num_centroids);
   for (int c0 = 0; c0 < num_centroids; c0 += kSortClusters)
     kmeans_range_emit_kernel<<<ranges, 32, smem, stream>>>(idx, w.range_hist, clusters, num_tokens, num_centroids, per_range, max_cluster_size, c0,
                                                            num_centroids - c0 < kSortClusters ? num_centroids - c0 : kSortClusters);
