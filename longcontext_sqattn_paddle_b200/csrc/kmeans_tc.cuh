@@ -28,9 +28,8 @@ constexpr int kKtTokens = 256;    // tokens per CTA (two M = 128 tiles)
 constexpr int kKtCent = 256;      // centroids per MMA group (N)
 constexpr int kKtStages = 2;
 // |tensor-core fp32 sum - exact| is bounded by (terms * 2^-22) * sum|terms| <= 2^-15 |k||x| for 128 terms; the two
-// scores that are compared each carry it, and the factor of two on top covers an accumulator that truncates.  The five
-// low bits that the epilogue spends on a score's column add 2^-18 |k||x| each.
-constexpr float kKtTol = 1.3e-4f;
+// scores that are compared each carry it, and the factor of two on top covers an accumulator that truncates
+constexpr float kKtTol = 1.25e-4f;
 
 struct KmeansTcParams {
   const uint8_t* data;      // [G, T, D] for the token norms
@@ -261,8 +260,10 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
       if (tok < p.num_tokens) {
         const long long at = static_cast<long long>(g) * p.num_tokens + tok;
         const int best_idx = best_chunk * 32 + static_cast<int>(__float_as_uint(best) & 31u);
-        const float tol = kKtTol * sqrtf(nrm2) * sqrtf(p.max_cnorm2[g]);
-        const bool sure = (best - second) > fmaxf(tol, 2e-38f);   // the columns of scores without a normal exponent are no order
+        // the accumulation's error, and what the columns in the low bits can make of equal scores (31 units in the last
+        // place; the norms may have underflowed, and scores without a normal exponent have coarser units still)
+        const float tol = kKtTol * sqrtf(nrm2) * sqrtf(p.max_cnorm2[g]) + 7.7e-6f * fabsf(best);
+        const bool sure = (best - second) > fmaxf(tol, 2e-38f);
         p.idx[at] = sure ? best_idx : (-1 - best_idx);
         if (!sure) {
           const int slot = atomicAdd(p.flagged_count, 1);

@@ -133,3 +133,30 @@ def test_member_sums_and_lists_with_uneven_clusters(dtype, t, d):
     for b in range(g):
         for c in range(k):
             assert torch.equal(lists[b, c, :n[b, c]].cpu().long(), (idx[b] == c).nonzero()[:, 0])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("g,t,k,d", [(1, 1, 32, 128), (2, 255, 96, 64), (3, 20001, 288, 128), (7, 6000, 544, 64)])
+def test_assignment_over_many_items(dtype, g, t, k, d):
+    """More 256-token items than CTAs, groups that end inside an item, centroid counts that end inside a tile.  Exact
+    arg-max: keys that are zero (every score ties, below any exponent), centroids that are repeated (lowest index), and a
+    NaN key, which has no arg-max but must get some centroid."""
+    from longcontext_sqattn_paddle_b200.cache_hub import kmeans as km
+    gen = torch.Generator(device="cuda").manual_seed(t)
+    data = torch.randn(g, t, d, generator=gen, device="cuda").to(dtype)
+    cent = torch.randn(g, k, d, generator=gen, device="cuda").to(dtype)
+    cent[:, k // 2:k // 2 + 8] = cent[:, :8]
+    data[:, ::7] = 0.0
+    data[:, 1::11] *= 1e-6 if dtype == torch.float16 else 1e-30
+    want = (data.double() @ cent.double().transpose(1, 2)).argmax(-1)
+    want[(data == 0).all(-1)] = 0
+    want = torch.where((want >= k // 2) & (want < k // 2 + 8), want - k // 2, want)
+    nan = t // 2
+    if t > 1:
+        data[0, nan, 3] = float("nan")
+    _, idx, counts = km.k_means_train(data, cent.clone(), True)
+    if t > 1:
+        assert 0 <= idx[0, nan].item() < k
+        want[0, nan] = idx[0, nan]
+    assert torch.equal(idx.long(), want)
+    assert torch.equal(counts.long(), torch.stack([torch.bincount(r.long(), minlength=k) for r in idx]))
