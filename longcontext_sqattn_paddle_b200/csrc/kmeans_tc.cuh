@@ -53,30 +53,26 @@ struct KmeansTcSmem {
   static constexpr int kTotal = kMiscOff + 16;
 };
 
-// max over the centroids of a group of sum_d x_d^2 (fp32): one CTA per group
+// max over the centroids of a group of sum_d x_d^2 (fp32); out is zeroed by the caller, and floats that are not negative
+// order like their bits.  D / 8 lanes per row, kCnormParts CTAs per group (one read its centroids row by row: 13 us).
+constexpr int kCnormParts = 8;
 template <int D, bool BF16>
 __global__ void __launch_bounds__(256) kmeans_cnorm_max_kernel(const uint8_t* cent, int num_centroids, float* out) {
-  __shared__ float red[8];
-  const int g = blockIdx.x;
-  const uint8_t* cg = cent + static_cast<long long>(g) * num_centroids * D * 2;
+  constexpr int kLanes = D / 8, kRows = 256 / kLanes;
+  const int g = blockIdx.x, c0 = blockIdx.y * kRows + threadIdx.x / kLanes, ch = threadIdx.x % kLanes;
+  const uint8_t* cg = cent + static_cast<long long>(g) * num_centroids * D * 2 + ch * 16;
   float m = 0.f;
-  for (int c = threadIdx.x; c < num_centroids; c += 256) {
-    float s = 0.f;
-    for (int ch = 0; ch < D / 8; ++ch) {
-      float f[8];
-      unpack8<BF16>(*reinterpret_cast<const uint4*>(cg + (static_cast<long long>(c) * D + ch * 8) * 2), f);
+  for (int c = c0; c < num_centroids; c += kCnormParts * kRows) {
+    float f[8], s = 0.f;
+    unpack8<BF16>(*reinterpret_cast<const uint4*>(cg + static_cast<long long>(c) * D * 2), f);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) s += f[i] * f[i];
-    }
+    for (int i = 0; i < 8; ++i) s += f[i] * f[i];
+    // the rows of a warp end together: num_centroids is a multiple of 32
+    for (int o = kLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     m = fmaxf(m, s);
   }
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 1; i < 8; ++i) m = fmaxf(m, red[i]);
-    out[g] = m;
-  }
+  if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(reinterpret_cast<int*>(out + g), __float_as_int(m));
 }
 
 template <int D>

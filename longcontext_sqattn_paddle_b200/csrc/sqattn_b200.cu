@@ -797,8 +797,9 @@ int sqattn_kmeans_assign(const void* data, const void* centroids, int32_t dtype,
   const bool bf16 = dtype == SQATTN_BF16;
   const uint8_t* d8 = static_cast<const uint8_t*>(data);
   const uint8_t* c8 = static_cast<const uint8_t*>(centroids);
-  SQ_CUDA(cudaMemsetAsync(w.flagged_count, 0, sizeof(int), stream));
-  SQ_KM_DISPATCH(kmeans_cnorm_max_kernel, <<<groups, 256, 0, stream>>>(c8, num_centroids, w.max_cnorm2));
+  // the norms and the flagged count lie next to each other
+  SQ_CUDA(cudaMemsetAsync(w.max_cnorm2, 0, reinterpret_cast<uint8_t*>(w.flagged_count + 1) - reinterpret_cast<uint8_t*>(w.max_cnorm2), stream));
+  SQ_KM_DISPATCH(kmeans_cnorm_max_kernel, <<<dim3(groups, kCnormParts), 256, 0, stream>>>(c8, num_centroids, w.max_cnorm2));
   if ((rc = head_dim == 128 ? km_launch_assign<128>(data, centroids, dtype, groups, num_tokens, num_centroids, idx, w, stream)
                             : km_launch_assign<64>(data, centroids, dtype, groups, num_tokens, num_centroids, idx, w, stream)))
     return rc;
