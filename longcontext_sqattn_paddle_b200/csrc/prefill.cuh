@@ -220,6 +220,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
   // once a wait has given up anywhere on this device, the remaining CTAs (and every later launch, until the host
   // has read and cleared the status word) only mark their rows as invalid
   if ((sbase & 1023u) || device_failed()) {
+    griddep_wait();
     poison_output<D>(p, bi, head, blk);
     return;
   }
@@ -259,6 +260,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_base_s;
+  griddep_wait();   // the set-up above may run while the kernel before this one drains
   const int nseg = *nseg_s;
   int nsteps = 0;
   for (int i = 0; i < nseg; ++i) nsteps += segs[i].ntiles;

@@ -30,13 +30,15 @@ double sm_scale_log2(int head_dim, int head_dim_og = 0) {
 // stream drains; the kernel itself waits (griddepcontrol.wait) before it reads anything an earlier kernel produced.
 // Which kernels get it is a measured choice (1M-token decode sharded over 2 GPUs, 28 layers per step, graph replay):
 // none 4.806 ms, the merge kernels only 4.800 ms, merge and decode kernels 5.245 ms (a decode grid that becomes
-// resident behind the running one slows it down), so only the merges do by default.
-// SQATTN_B200_OVERLAP (read once) overrides with a bit mask of kernel classes: 1 = merge kernels, 2 = decode kernel.
+// resident behind the running one slows it down), so of those only the merges do by default.  The operator's preparation
+// and its attention kernel do: 8192 tokens, FP8 P: 280 us a call with, 293 without.
+// SQATTN_B200_OVERLAP (read once) overrides with a bit mask of kernel classes: 1 = merge kernels, 2 = decode kernel,
+// 4 = preparation and prefill kernels.
 int overlap_mask() {
   static int mask = -1;
   if (mask < 0) {
     const char* e = getenv("SQATTN_B200_OVERLAP");
-    mask = (e && e[0] >= '0' && e[0] <= '3') ? e[0] - '0' : 1;
+    mask = (e && e[0] >= '0' && e[0] <= '7') ? e[0] - '0' : 5;
   }
   return mask;
 }
@@ -204,7 +206,7 @@ int launch_prefill(const sqattn_prefill_args* a, const PrefillPlan& pl, cudaStre
     using L = PrefillSmem<D, 2, 3>;   /* two K stages (tied to the two S buffers), three V stages, two CTAs per SM */    \
     auto kernel = prefill_kernel<D, DUMP, 2, 3, 2, FP8>;                                                                 \
     SQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynBytes));                    \
-    kernel<<<static_cast<unsigned>(grid), 192, L::kDynBytes, stream>>>(tq8, tq4, tk8, tk4, tv, p);                       \
+    SQ_CUDA(launch_overlapped(4, kernel, dim3(static_cast<unsigned>(grid)), dim3(192), L::kDynBytes, stream, tq8, tq4, tk8, tk4, tv, p)); \
   } while (0)
   if (dump || dump_t || dump_p) SQ_LAUNCH_PREFILL(true, true);
   else if (a->p_fp8_mode) SQ_LAUNCH_PREFILL(false, true);
@@ -593,35 +595,33 @@ int sqattn_prep_qkv(const sqattn_prep_args* a, sqattn_stream_t stream_) {
   const int B = a->batch, N = a->seq_len, D = a->head_dim, Hq = a->num_q_heads, Hkv = a->num_kv_heads;
   const bool bf16 = a->dtype == SQATTN_BF16;
   float* partial = static_cast<float*>(a->workspace);
-  float* mean_ws = partial + static_cast<size_t>(B) * Hkv * kMeanChunks * D;
   View4 kq = view_of(a->q, B, Hq, N, D), kk = view_of(a->k, B, Hkv, N, D), kv = view_of(a->v, B, Hkv, N, D);
   const float* mean = a->k_mean;
-  if (!mean && do_k) {
-    const int lanes = 256 / (D / 8);
-    dim3 mg(kMeanChunks, B * Hkv);
-    if (bf16) kmean_partial_kernel<true><<<mg, 256, lanes * D * sizeof(float), stream>>>(kk, partial);
-    else kmean_partial_kernel<false><<<mg, 256, lanes * D * sizeof(float), stream>>>(kk, partial);
-    kmean_final_kernel<<<B * Hkv, 128, 0, stream>>>(partial, mean_ws, D, N);
-    mean = mean_ws;
-  }
   const float qs = static_cast<float>(sm_scale_log2(D));
-  uint8_t* q4 = a->skip_bit4 ? nullptr : static_cast<uint8_t*>(a->q_bit4);
-  uint8_t* k4 = a->skip_bit4 ? nullptr : static_cast<uint8_t*>(a->k_bit4);
   const OutStrides qo{static_cast<long long>(Hq) * N * D, static_cast<long long>(N) * D, D};
   const OutStrides ko = a->kv_out_nhd ? OutStrides{static_cast<long long>(N) * Hkv * D, D, static_cast<long long>(Hkv) * D}
                                       : OutStrides{static_cast<long long>(Hkv) * N * D, static_cast<long long>(N) * D, D};
-  const int rows_per_block = 256 / (D / 8);
-  const int gx = elementwise_grid((N + 4 * rows_per_block - 1) / (4 * rows_per_block), 1);
-  const dim3 gq(gx, B * Hq), gk(gx, B * Hkv);
-  const int gv = elementwise_grid(static_cast<long long>(N) * (D / 8), 256);
-  if (bf16) {
-    if (do_q) quant_rows_kernel<true, false><<<gq, 256, 0, stream>>>(kq, nullptr, static_cast<uint8_t*>(a->q_bit8), q4, qo, a->qk_qtype, a->round_half_even, qs);
-    if (do_k) quant_rows_kernel<true, true><<<gk, 256, 0, stream>>>(kk, mean, static_cast<uint8_t*>(a->k_bit8), k4, ko, a->qk_qtype, a->round_half_even, 1.0f);
-    if (do_v) quant_v_kernel<true><<<gv, 256, 0, stream>>>(kv, static_cast<uint8_t*>(a->v_bit8), ko, a->v_qtype, a->round_half_even);
-  } else {
-    if (do_q) quant_rows_kernel<false, false><<<gq, 256, 0, stream>>>(kq, nullptr, static_cast<uint8_t*>(a->q_bit8), q4, qo, a->qk_qtype, a->round_half_even, qs);
-    if (do_k) quant_rows_kernel<false, true><<<gk, 256, 0, stream>>>(kk, mean, static_cast<uint8_t*>(a->k_bit8), k4, ko, a->qk_qtype, a->round_half_even, 1.0f);
-    if (do_v) quant_v_kernel<false><<<gv, 256, 0, stream>>>(kv, static_cast<uint8_t*>(a->v_bit8), ko, a->v_qtype, a->round_half_even);
+  // first launch: column sums of K and all of V
+  const int sum_blocks = do_k && !mean ? kMeanChunks * B * Hkv : 0;
+  const int v_blocks = do_v ? elementwise_grid(static_cast<long long>(N) * (D / 4), 256) : 0;
+  if (sum_blocks + v_blocks > 0) {
+    const bool vint = a->v_qtype == SQATTN_QTYPE_INT;
+    auto sums_v = bf16 ? (vint ? prep_sums_v_kernel<true, true> : prep_sums_v_kernel<true, false>) : (vint ? prep_sums_v_kernel<false, true> : prep_sums_v_kernel<false, false>);
+    sums_v<<<sum_blocks + v_blocks, 256, 0, stream>>>(kk, partial, sum_blocks, kv, static_cast<uint8_t*>(a->v_bit8), ko, a->v_qtype, a->round_half_even);
+    SQ_CUDA(cudaGetLastError());
+  }
+  // second launch: rows of Q and K, 64 (D = 128) or 128 rows of one head per block
+  if (do_q || do_k) {
+    const int rows = kQuantRowsPerThread * 256 / (D / 8), blocks = (N + rows - 1) / rows;
+    QuantRows q{kq, static_cast<uint8_t*>(a->q_bit8), a->skip_bit4 ? nullptr : static_cast<uint8_t*>(a->q_bit4), qo, blocks};
+    QuantRows k{kk, static_cast<uint8_t*>(a->k_bit8), a->skip_bit4 ? nullptr : static_cast<uint8_t*>(a->k_bit4), ko, blocks};
+    const int q_blocks = do_q ? q.blocks * B * Hq : 0, k_blocks = do_k ? k.blocks * B * Hkv : 0;
+    const dim3 grid(q_blocks + k_blocks);
+    const int klass = sum_blocks + v_blocks > 0 ? 4 : 0;   // its query blocks read ahead of the wait: only behind the launch above
+    const bool grid8 = a->qk_qtype == SQATTN_QTYPE_INT;
+    auto rows_kernel = bf16 ? (grid8 ? prep_rows_kernel<true, true> : prep_rows_kernel<true, false>)
+                            : (grid8 ? prep_rows_kernel<false, true> : prep_rows_kernel<false, false>);
+    SQ_CUDA(launch_overlapped(klass, rows_kernel, grid, dim3(256), 0, stream, q, k, q_blocks, partial, mean, a->qk_qtype, a->round_half_even, qs));
   }
   SQ_CUDA(cudaGetLastError());
   return SQATTN_OK;

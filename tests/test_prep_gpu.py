@@ -129,3 +129,22 @@ def test_q_fake_quant_inside_the_attention_kernel_is_bit_identical(dtype, qtype)
         ops.prefill(query, k8, q8.permute(0, 2, 1, 3), k8, v8, layout="NHD", kv_layout="HND", q_fake_quant=qtype, **kw)
     torch.cuda.synchronize()
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("n,hq,hkv,d", [(1, 4, 2, 128), (63, 4, 1, 64), (8257, 28, 4, 128), (20011, 32, 8, 128), (16500, 32, 8, 64)])
+def test_prep_rounds_of_rows(n, hq, hkv, d):
+    """Rows are independent given K's mean, so a call whose blocks go over several rounds of rows equals calls on short
+    slices, whose blocks take one, bit for bit; so do calls that prepare one tensor at a time."""
+    from longcontext_sqattn_paddle_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(n)
+    qkv = torch.randn(1, n, (hq + 2 * hkv) * d, generator=g, device="cuda", dtype=torch.bfloat16)
+    q, k, v = (t.view(1, n, -1, d) for t in qkv.split([hq * d, hkv * d, hkv * d], dim=-1))
+    whole = ops.prep_qkv(q, k, v)
+    mean = ops.k_column_sums(k) / torch.tensor(float(n), device="cuda")
+    step = 1000
+    for r in range(0, n, step):
+        part = ops.prep_qkv(q[:, r:r + step], k[:, r:r + step], v[:, r:r + step], k_mean=mean)
+        for w, p in zip(whole, part):
+            assert torch.equal(w[:, :, r:r + step], p)
+    one = ops.prep_qkv(q, None, None)[:2] + ops.prep_qkv(None, k, None)[2:4] + ops.prep_qkv(None, None, v)[4:]
+    assert all(torch.equal(w, o) for w, o in zip(whole, one))
