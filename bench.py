@@ -555,7 +555,8 @@ def run_ours(args):
         spfn = sqdist.sp_prefill_wrapper(r, r, SINK, _Args(), seq_total=n_total, layout="balanced")
         op = lambda q, k, v: spfn(_Layer(), q, k, v, None)
         segs = sqdist.ShardLayout.balanced(n_total, world, w, SINK).segments(rank)
-    launches_per_step = 6   # column sums (2), quantise V, K and Q, attention
+    # column sums of K with V, rows of Q and K, attention; sharded: column sums (2), V, K and Q by themselves, attention
+    launches_per_step = 3 if world == 1 else 6
     ns = sum(hi - lo for lo, hi in segs)
 
     # synthetic input: this rank's rows of the sequence, resident in HBM and mirrored in pinned host memory
