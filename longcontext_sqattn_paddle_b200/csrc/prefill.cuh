@@ -19,7 +19,6 @@ constexpr int kBlockM = 128;  // query rows per CTA (tcgen05 M)
 constexpr int kBlockN = 64;   // keys per step (the reference BLOCK_N)
 constexpr int kMaxSegs = 12;
 constexpr float kLazyLog2 = 8.0f;  // O is rescaled only when a row's maximum has moved by more than 2^8
-constexpr float kFp8Lead = 8.0f;   // kernels with an FP8 P: how far the reference of P, l and O starts below the maximum
 
 // segment flags
 constexpr int kSegAct0 = 1;   // rows 0..63 of the CTA take part
@@ -447,7 +446,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
       tc_fence_after();
       if (warp == 2 && lane == 0) SQ_STAMP(i, 6);
       uint32_t pk[32];
-      float alpha = 1.0f, to_base = 1.0f;
+      float alpha = 1.0f;
       if (flags & half_bit) {
         uint32_t r0[32], r1[32];
         tmem_ld32(s_tmem, r0);
@@ -478,17 +477,15 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
         // P, l and O are kept relative to `base`, which follows the running maximum only when it has moved by
         // more than kLazyLog2 (so P <= 2^kLazyLog2): O then needs its rescale (a wait for the previous P V plus a
         // TMEM round trip) a few times per row instead of whenever the maximum moves.  Steps whose P is rounded
-        // through e4m3 round p = 2^(s - running maximum), as the rule says, and bring the rounded value to `base` with
-        // the factor 2^(m - base) in the multiplication that takes the 448 off again: still one rounding to f16.  There
-        // base stays kFp8Lead below the maximum it was set to, which keeps the smallest e4m3 values among f16's normal
-        // numbers (P <= 2^15).
-        if (m_new > base + (kFp8 ? kLazyLog2 + kFp8Lead - 1.0f : kLazyLog2)) {
-          const float to = kFp8 ? m_new - kFp8Lead : m_new;
-          alpha = ex2_approx(base - to);
-          base = to;
+        // through e4m3 keep base == running maximum: p <= 1 as the rounding rule expects, and P is f16(e4m3(448 p) / 448)
+        // itself.  (A lazy base there has to bring P to it by the factor 2^(m - base), which is no power of two: 8192
+        // tokens took 27 us less, but the f16 rounding of the scaled P lost the exact P = 1 of the row's maximum and was
+        // a tenth larger on average.)
+        if (m_new > base + (fp8 ? 0.0f : kLazyLog2)) {
+          alpha = ex2_approx(base - m_new);
+          base = m_new;
         }
-        const float p_ref = fp8 ? m_new : base;
-        const uint64_t m2 = f32x2_pack(p_ref, p_ref);
+        const uint64_t m2 = f32x2_pack(base, base);
         uint64_t sa = f32x2_pack(0.0f, 0.0f), sb = sa;
 #pragma unroll
         for (int c = 0; c < 64; c += 4) {
@@ -502,17 +499,13 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
         float s0, s1, s2, s3;
         f32x2_unpack(sa, s0, s1);
         f32x2_unpack(sb, s2, s3);
-        float sum = (s0 + s1) + (s2 + s3);
-        if (fp8) { to_base = ex2_approx(m_new - base); sum *= to_base; }
+        const float sum = (s0 + s1) + (s2 + s3);
         l_i = l_i * alpha + sum;
         if (warp == 2 && lane == 0) SQ_STAMP(i, 9);
         m_i = m_new;
         if (fp8) {
-          const float f = to_base * (1.0f / 448.0f);
-          const __half fh = __float2half_rn(f), fl = __float2half_rn(f - __half2float(fh));
-          const __half2 hi = __half2half2(fh), lo = __half2half2(fl);
 #pragma unroll
-          for (int c = 0; c < 32; ++c) pk[c] = p_fp8_times(x[2 * c], x[2 * c + 1], hi, lo);
+          for (int c = 0; c < 32; ++c) pk[c] = p_fp8_round_f16x2(x[2 * c], x[2 * c + 1]);
         } else {
 #pragma unroll
           for (int c = 0; c < 32; ++c) pk[c] = pack_f16x2(x[2 * c], x[2 * c + 1]);
@@ -526,7 +519,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
         for (int c = 0; c < 32; ++c) {
           const __half2 h = *reinterpret_cast<const __half2*>(&pk[c]);
           float* dst = p.dump_p + (static_cast<size_t>(i) * kBlockM + row_in_tile) * 64 + 2 * c;
-          dst[0] = __low2float(h) / to_base; dst[1] = __high2float(h) / to_base;   // relative to the step's maximum
+          dst[0] = __low2float(h); dst[1] = __high2float(h);
         }
       }
       tmem_st32(s_tmem, pk);

@@ -1,7 +1,6 @@
 // Thin inline-PTX wrappers for the sm_100a features the kernels use:
 // mbarrier, TMA tiled loads (cp.async.bulk.tensor), tcgen05 MMA / TMEM.
 #pragma once
-#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -320,22 +319,6 @@ __device__ __forceinline__ uint32_t p_fp8_round_f16x2(float lo, float hi) {
       : "r"(h2));
   const float inv = 1.0f / 448.0f;
   return pack_f16x2(flo * inv, fhi * inv);
-}
-
-// f16(e4m3(448 p) * f) for two p in [0, 1], f = hi + lo >= 0.5 in two f16 parts (lo: what f16 takes off f).  Rounding
-// the small product first adds at most a thirtieth of the last place to the one rounding of the result (its error is
-// 2^-25 where the smallest e4m3 value's product has steps of 2^-20).  Two instructions for two values behind the
-// conversions, where unpacking to fp32 takes five.
-__device__ __forceinline__ uint32_t p_fp8_times(float p_lo, float p_hi, __half2 hi, __half2 lo) {
-  float t0, t1;
-  f32x2_unpack(f32x2_mul(f32x2_pack(p_lo, p_hi), f32x2_pack(448.0f, 448.0f)), t0, t1);
-  uint16_t e;
-  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(e) : "f"(t1), "f"(t0));
-  uint32_t h2;
-  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"(e));
-  const __half2 v = *reinterpret_cast<const __half2*>(&h2);
-  const __half2 r = __hfma2(v, hi, __hmul2(v, lo));
-  return *reinterpret_cast<const uint32_t*>(&r);
 }
 
 }  // namespace sq

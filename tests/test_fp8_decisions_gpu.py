@@ -40,8 +40,8 @@ def _e4m3_codes(p):
     return (p * 448.0).to(torch.float8_e4m3fn).view(torch.uint8)
 
 
-@pytest.mark.parametrize("mode,sink,w8,w4", [(0, 0, 0, 0), (2, 64, 300, 520)])
-def test_fp8_rounding_decisions_of_p(dbg, mode, sink, w8, w4):
+def _dump(dbg, mode, sink, w8, w4):
+    """Scaled queries, keys, the first CTA's query block, its steps (first key, flags) and the S and P tiles of each step."""
     from longcontext_sqattn_paddle_b200 import _lib as L, ops
     n, hq, hkv, d, dtype = 1536, 2, 1, 128, torch.bfloat16
     g = torch.Generator().manual_seed(41)
@@ -70,7 +70,12 @@ def test_fp8_rounding_decisions_of_p(dbg, mode, sink, w8, w4):
     rc = dbg.sqattn_debug_prefill_dump_sp(C.byref(a), dump_s.data_ptr(), dump_p.data_ptr(), torch.cuda.current_stream().cuda_stream)
     assert rc == 0, dbg.sqattn_last_error_string()
     torch.cuda.synchronize()
-    s_k, p_k = dump_s.cpu(), dump_p.cpu()
+    return qs, k, blk, steps, dump_s.cpu(), dump_p.cpu()
+
+
+@pytest.mark.parametrize("mode,sink,w8,w4", [(0, 0, 0, 0), (2, 64, 300, 520)])
+def test_fp8_rounding_decisions_of_p(dbg, mode, sink, w8, w4):
+    qs, k, blk, steps, s_k, p_k = _dump(dbg, mode, sink, w8, w4)
     rows = torch.arange(blk * 128, blk * 128 + 128)
     qrow = qs[0, 0, rows].float()
     m_own = torch.full((128,), float("-inf"))
@@ -98,3 +103,12 @@ def test_fp8_rounding_decisions_of_p(dbg, mode, sink, w8, w4):
     assert far == 0
     assert f_own < 2e-3, f_own
     assert f_ref < 2e-2, f_ref
+
+
+@pytest.mark.parametrize("mode,sink,w8,w4", [(0, 0, 0, 0), (2, 64, 300, 520)])
+def test_p_reaches_the_product_with_the_reference_bits(dbg, mode, sink, w8, w4):
+    """Whatever the codes, the f16 value that P V multiplies is f16(code / 448) exactly (attn_triton.py:81-83)."""
+    *_, p_k = _dump(dbg, mode, sink, w8, w4)
+    value = _e4m3_codes(p_k).view(torch.float8_e4m3fn).double() / 448.0
+    assert torch.equal(p_k, value.half().float())
+    assert (p_k == 1.0).any() and p_k.max() == 1.0        # a row's maximum is exact
