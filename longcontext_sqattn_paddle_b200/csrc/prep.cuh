@@ -269,16 +269,16 @@ __device__ __forceinline__ void quant_v_body(const View4& v, uint8_t* out, const
   auto store = [&](const uint2& r, long long off) {
     float f[4], g[4];
     unpack4(r, f);
-    float worst = kInt ? 0.f : 1.0f;
-    if (kInt) {   // the reciprocal and its check: see fake_quant_int_row8
+    bool sure = kInt;
+    if (kInt) {   // the reciprocal and its check: see fake_quant_int_row8; a NaN is never sure, the clamp decides about it
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float q = f[i] * inv[i], rq = rintf(q);
-        worst = fmaxf(worst, fabsf(q - rq));
+        sure = sure && fabsf(q - rq) <= 0.4999f;
         g[i] = rq * scale[i];
       }
     }
-    if (worst > 0.4999f) {
+    if (!sure) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) g[i] = fake_quant_value(f[i], amax[i], qtype, 127.0f, half_even);
     }

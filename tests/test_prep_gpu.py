@@ -148,3 +148,24 @@ def test_prep_rounds_of_rows(n, hq, hkv, d):
             assert torch.equal(w[:, :, r:r + step], p)
     one = ops.prep_qkv(q, None, None)[:2] + ops.prep_qkv(None, k, None)[2:4] + ops.prep_qkv(None, None, v)[4:]
     assert all(torch.equal(w, o) for w, o in zip(whole, one))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_a_nan_in_v_ends_on_the_lowest_step_whatever_lies_beside_it(dtype):
+    """The clamp of the integer grid turns a NaN into -128 steps of its channel (the range is taken over the other heads),
+    also where none of the channels that one thread holds sits near a half.  The other values are what they are without it."""
+    from longcontext_sqattn_paddle_b200 import ops
+    g = torch.Generator().manual_seed(5)
+    v = torch.randn(1, 200, 6, 64, generator=g).to(dtype)
+    heads, chans = torch.arange(200) % 6, torch.arange(200) * 7 % 64
+    at = (0, torch.arange(200), heads, chans)
+    zero = v.clone()
+    zero[at] = 0.0                                        # a zero leaves the range to the other heads as a NaN does
+    bad = v.clone()
+    bad[at] = float("nan")
+    want, got = (ops.prep_qkv(None, None, t.cuda())[4].cpu().transpose(1, 2) for t in (zero, bad))
+    step = (zero.float().abs().amax((0, 2)).clamp_min(1e-5) / 127.0)[torch.arange(200), chans]
+    assert torch.equal(got[at], (step * -128.0).to(dtype).to(torch.float16))
+    want, got = want.clone(), got.clone()
+    want[at] = got[at] = 0.0
+    assert torch.equal(want, got)
