@@ -198,6 +198,8 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         for (int e = 0; e < 8; ++e) acc[e] += f[e];
       }
     }
+    // this warp has read its last tile (or given up): the consumers, who write the merge scratch over the ring, wait for it
+    asm volatile("bar.arrive 1, 256;" ::: "memory");
     float* col = reinterpret_cast<float*>(smem + L::kSumOff);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
@@ -407,7 +409,9 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       l_r[r] += __shfl_xor_sync(0xffffffffu, l_r[r], 1);
       l_r[r] += __shfl_xor_sync(0xffffffffu, l_r[r], 2);
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");  // all consumer warps are done with the ring
+    // all warps that read the ring are done with it: the four consumers, and the four that add up columns
+    if (kColSum) asm volatile("bar.sync 1, 256;" ::: "memory");
+    else asm volatile("bar.sync 1, 128;" ::: "memory");
     float* scratch = reinterpret_cast<float*>(smem);
     float* my = scratch + warp * (16 * D + 32);
 #pragma unroll
@@ -422,7 +426,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     }
     asm volatile("bar.sync 1, 128;" ::: "memory");
     // the abort flag is stable here: the producer has issued its last copy before the consumers pass the last
-    // full barrier, and a consumer that gave up did so before the barrier above
+    // full barrier, and a reader of the ring that gave up did so before the barriers above
     if (*cta_abort) {
       poison_partials(128);
     } else if (ok) {

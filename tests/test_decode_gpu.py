@@ -199,3 +199,22 @@ def test_centred_decode_keeps_the_copy_where_it_has_to():
     k2[0, 1, 7, 5] = float("inf")
     o = attn_unified(q, k2, v, "HND", dtype)
     assert torch.isnan(o[0, 4:]).all() and torch.isfinite(o[0, :4]).all() and torch.isfinite(o[1]).all()
+
+
+@pytest.mark.parametrize("b,hq,hkv,L,d", [(1, 28, 4, 129, 128), (1, 8, 8, 193, 64), (2, 32, 8, 3001, 128), (1, 28, 4, 70001, 128)])
+def test_centred_decode_repeats_itself(b, hq, hkv, L, d):
+    """The column sums are taken from tiles whose shared memory is reused for the merge of the warps: the same call gives
+    the same bits every time, and the mean shows in every LSE (keys with an offset, a last tile that is not full)."""
+    from longcontext_sqattn_paddle_b200.sqattn import attn_unified
+    dtype = torch.bfloat16
+    q, k, v = (_rand(s, L + i, dtype).cuda() for i, s in enumerate([(b, hq, 1, d), (b, hkv, L, d), (b, hkv, L, d)]))
+    k += 2.0
+    first = attn_unified(q, k, v, "HND", dtype, True)
+    for _ in range(200):
+        o, lse = attn_unified(q, k, v, "HND", dtype, True)
+        assert torch.equal(o, first[0]) and torch.equal(lse, first[1])
+    qs = (q.float() * np.float32(1.0 / d ** 0.5 * 1.44269504)).to(dtype).double()
+    kc = (k.double() - k.double().mean(dim=2, keepdim=True).to(dtype).double()).repeat_interleave(hq // hkv, 1)
+    s = torch.cat([qs @ kc.transpose(2, 3), torch.zeros(b, hq, 1, -L % 64, dtype=torch.float64, device="cuda")], -1)
+    rlse = torch.logsumexp(s * np.log(2.0), -1) / np.log(2.0)
+    assert (first[1].double() - rlse).abs().max().item() < 1e-3        # as above: fp32 sums of scores up to 100
