@@ -132,7 +132,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       if (idx % D == 0) p.part_lse[orow] = nan;
     }
   };
-  if (device_failed()) {
+  if (cta_device_failed()) {
     poison_partials(blockDim.x);
     return;
   }

@@ -96,7 +96,7 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
     }
     if (threadIdx.x == 0) atomicMax(p.flagged_count, p.flagged_cap + 1);   // forces the full sweep
   };
-  if ((sbase & 1023u) || device_failed()) {
+  if ((sbase & 1023u) || cta_device_failed()) {
     if ((sbase & 1023u) && threadIdx.x == 0) record_failure(400);
     mark_for_recheck(blockIdx.x);
     return;

@@ -218,7 +218,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
   if ((sbase & 1023u) && threadIdx.x == 0) record_failure(100);
   // once a wait has given up anywhere on this device, the remaining CTAs (and every later launch, until the host
   // has read and cleared the status word) only mark their rows as invalid
-  if ((sbase & 1023u) || device_failed()) {
+  if ((sbase & 1023u) || cta_device_failed()) {
     griddep_wait();
     poison_output<D>(p, bi, head, blk);
     return;

@@ -61,6 +61,10 @@ __device__ __forceinline__ void record_failure(int code) {
 }
 __device__ __forceinline__ bool device_failed() { return *reinterpret_cast<volatile int*>(&g_device_status) != 0; }
 
+// The same for a whole CTA, one answer for all of its threads: the word may be set while they read it, and a warp that left
+// alone would miss at the barriers (or leave them, and the tensor memory, uninitialised for the others).
+__device__ __forceinline__ bool cta_device_failed() { return __syncthreads_or(device_failed()) != 0; }
+
 constexpr uint64_t kWaitLimitNs = 1000000000ull;  // every device-side wait gives up after one second
 
 // Bounded wait.  Returns false after kWaitLimitNs (or as soon as another thread

@@ -214,7 +214,7 @@ window_hist_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   auto poison = [&]() {   // this CTA cannot deliver its rows
     for (int b = threadIdx.x; b < p.nbins; b += blockDim.x) atomicAdd(out + b, __longlong_as_double(0x7ff8000000000000ll));
   };
-  if ((sbase & 1023u) || device_failed()) {
+  if ((sbase & 1023u) || cta_device_failed()) {
     if ((sbase & 1023u) && threadIdx.x == 0) record_failure(500);
     poison();
     return;
