@@ -263,7 +263,9 @@ struct DecodePlan {
 // 79; 3 of 20000 52 and 48.5; beyond two CTAs per SM a second wave costs more than it evens out (121, 77, 96, 60).
 // Keys through an index list: two per SM as well, since the warps' own chain per tile bounds the kernel there (64 lists
 // of 4096 keys, FP8 P: 51 and 36 us; 56: 43 and 30; 16: 20 and 17).
-int plan_decode(const sqattn_decode_args* a, DecodePlan* pl) {
+// The kernel that also adds up columns (centred) has 320 threads of more than 150 registers, so one CTA fits on an SM and
+// anything beyond 148 CTAs is a second wave.
+int plan_decode(const sqattn_decode_args* a, DecodePlan* pl, bool centered = false) {
   if (!a) return fail(SQATTN_ERR_INVALID_ARG, "args is null");
   if (a->head_dim != 64 && a->head_dim != 128) return fail(SQATTN_ERR_UNSUPPORTED, "head_dim %d: only 64 and 128", a->head_dim);
   if (a->batch <= 0 || a->batch > kDecMaxBatch) return fail(SQATTN_ERR_UNSUPPORTED, "batch must be in [1, %d]", kDecMaxBatch);
@@ -299,8 +301,8 @@ int plan_decode(const sqattn_decode_args* a, DecodePlan* pl) {
   } else {
     const long long target = (148ll + a->num_kv_heads - 1) / a->num_kv_heads;  // items per KV head
     chunk = static_cast<int>((total_tiles + target - 1) / target) * kDecTile;
-    const long long most = (a->gather || a->batch > 8 ? 296ll : 222ll) / a->num_kv_heads;
-    if ((a->batch > 1 || a->gather) && most > a->batch && total_tiles > 0) {
+    const long long most = (centered ? 148ll : a->gather || a->batch > 8 ? 296ll : 222ll) / a->num_kv_heads;
+    if ((a->batch > 1 || a->gather || centered) && most > a->batch && total_tiles > 0) {
       auto items_of = [&](long long c) {
         long long n = 0;
         for (int b = 0; b < a->batch; ++b) n += (pl->lens[b] + c - 1) / c;
@@ -655,7 +657,7 @@ size_t sqattn_decode_workspace_bytes(const sqattn_decode_args* args) {
 
 static int decode_impl(const sqattn_decode_args* a, cudaStream_t stream, bool centered) {
   DecodePlan pl;
-  int rc = plan_decode(a, &pl);
+  int rc = plan_decode(a, &pl, centered);
   if (rc) return rc;
   if (!a->q.ptr || (!a->gather && (!a->k.ptr || !a->v.ptr))) return fail(SQATTN_ERR_INVALID_ARG, "null tensor pointer");
   if (!a->partial_o && !a->o.ptr && !a->peer) return fail(SQATTN_ERR_INVALID_ARG, "null output pointer");
@@ -690,7 +692,7 @@ static int centered_check(const sqattn_decode_args* a) {
 
 size_t sqattn_decode_centered_workspace_bytes(const sqattn_decode_args* a) {
   DecodePlan pl;
-  if (centered_check(a) || plan_decode(a, &pl)) return 0;
+  if (centered_check(a) || plan_decode(a, &pl, true)) return 0;
   return decode_ws_bytes(a, pl) + decode_ksum_bytes(a, pl);
 }
 

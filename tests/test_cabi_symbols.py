@@ -50,3 +50,16 @@ def test_struct_layout_matches_header():
     assert L.PrefillArgs.lse.offset == 6 * 32
     assert L.PrefillArgs.win8_ratios.offset == 6 * 32 + 8 + 12 * 4
     assert L.DecodeArgs.kv_lens.offset == 4 * 32 + 8 + 6 * 4
+
+
+@pytest.mark.parametrize("batch,n,hq,hkv", [(1, 32000, 28, 4), (1, 32000, 32, 8), (1, 100000, 24, 3), (2, 32000, 28, 4), (2, 100000, 28, 4),
+                                            (3, 5000, 32, 8), (16, 20000, 28, 4)])
+def test_centred_decode_is_planned_for_one_cta_per_sm(batch, n, hq, hkv):
+    """Its CTAs are too large for two on an SM, so a launch of more than 148 takes two waves.  The workspace size tells the
+    number of work items: an item has a partial row and an LSE per query head and the column sums of every KV head."""
+    from longcontext_sqattn_paddle_b200 import _lib as L
+    d = 128
+    a = L.DecodeArgs()
+    a.batch, a.num_q_heads, a.num_kv_heads, a.head_dim, a.kv_len, a.dtype = batch, hq, hkv, d, n, L.BF16
+    items = L.lib.sqattn_decode_centered_workspace_bytes(C.byref(a)) // (4 * (hq * d + hq + hkv * d))   # padding is below one item
+    assert 0.75 * min(148, hkv * batch * -(-n // 256)) <= items * hkv <= 148
