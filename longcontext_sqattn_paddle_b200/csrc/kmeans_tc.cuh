@@ -15,7 +15,8 @@
 //
 // Exactness: the fp32 tensor-core score is not the exact inner product, so a token whose best and second-best
 // scores are closer than a bound on that error is put on a list and re-scored in fp64 by kmeans_recheck_list_kernel
-// (exact products, index-order sum, lowest index on ties): the final assignment is the exact argmax.
+// (exact products, index-order sum, lowest index on ties): the final assignment is the exact argmax.  The bound is a
+// product of norms; where one of them is too small for an fp32 square there is no bound and every centroid is re-scored.
 #pragma once
 #include <cuda.h>
 
@@ -30,6 +31,9 @@ constexpr int kKtStages = 2;
 // |tensor-core fp32 sum - exact| is bounded by (terms * 2^-22) * sum|terms| <= 2^-15 |k||x| for 128 terms; the two
 // scores that are compared each carry it, and the factor of two on top covers an accumulator that truncates
 constexpr float kKtTol = 1.25e-4f;
+// Squared norms from here on (2^-100) bound the error as stated: squares and products that underflow are below 2^-126 each,
+// less than 2^-119 in all, where the bound is at least 1.25e-4 * 2^-100 = 2^-113.
+constexpr float kKtMinNorm2 = 7.888609e-31f;
 
 struct KmeansTcParams {
   const uint8_t* data;      // [G, T, D] for the token norms
@@ -257,9 +261,9 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
         const long long at = static_cast<long long>(g) * p.num_tokens + tok;
         const int best_idx = best_chunk * 32 + static_cast<int>(__float_as_uint(best) & 31u);
         // the accumulation's error, and what the columns in the low bits can make of equal scores (31 units in the last
-        // place; the norms may have underflowed, and scores without a normal exponent have coarser units still)
+        // place of each)
         const float tol = kKtTol * sqrtf(nrm2) * sqrtf(p.max_cnorm2[g]) + 7.7e-6f * fabsf(best);
-        const bool sure = (best - second) > fmaxf(tol, 2e-38f);
+        const bool sure = (best - second) > tol && fminf(nrm2, p.max_cnorm2[g]) >= kKtMinNorm2;
         p.idx[at] = sure ? best_idx : (-1 - best_idx);
         if (!sure) {
           const int slot = atomicAdd(p.flagged_count, 1);
@@ -286,7 +290,7 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
 //   1. fp32 scores of ALL centroids of the group into shared memory, a half warp (D = 128) per centroid row with
 //      16-byte loads, so a token costs one coalesced sweep over its group's centroids;
 //   2. the candidates: centroids whose fp32 score lies within the error band of the largest one (the same bound
-//      as in the assignment kernel, which also covers this pass's own rounding);
+//      as in the assignment kernel, which also covers this pass's own rounding); a score that is not a number counts;
 //   3. the candidates' exact scores in fp64 (exact products, index-order sum), the largest wins, the lowest index
 //      on ties.  More than kMaxCand candidates (degenerate data, e.g. an all-zero key) take the fp64 path for every
 //      centroid.
@@ -372,10 +376,11 @@ kmeans_recheck_list_kernel(const uint8_t* data, const uint8_t* cent, int* idx, c
     __syncthreads();
     mx = red_s[0];
     for (int w = 1; w < 8; ++w) mx = fmaxf(mx, red_s[w]);
-    // 2. candidates inside the error band
-    const float tol = kKtTol * sqrtf(nrm2) * sqrtf(max_cnorm2[g]);
+    // 2. candidates inside the error band; without a band (norms beyond fp32 squares either way) none is left out
+    const float cnorm2 = max_cnorm2[g];
+    const float tol = fminf(nrm2, cnorm2) >= kKtMinNorm2 ? kKtTol * sqrtf(nrm2) * sqrtf(cnorm2) : INFINITY;
     for (int c = threadIdx.x; c < num_centroids; c += 256) {
-      if (score_s[c] >= mx - tol) {
+      if (!(score_s[c] < mx - tol)) {
         const int slot = atomicAdd(&ncand_s, 1);
         if (slot < kMaxCand) cand_s[slot] = c;
       }

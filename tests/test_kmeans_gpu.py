@@ -160,3 +160,28 @@ def test_assignment_over_many_items(dtype, g, t, k, d):
         want[0, nan] = idx[0, nan]
     assert torch.equal(idx.long(), want)
     assert torch.equal(counts.long(), torch.stack([torch.bincount(r.long(), minlength=k) for r in idx]))
+
+
+@pytest.mark.parametrize("key_exp,cent_exp", [(0, 0), (-90, 0), (0, -90), (-80, -70), (100, 30)])
+@pytest.mark.parametrize("d", [64, 128])
+def test_assignment_where_fp32_has_no_squares_of_the_norms(d, key_exp, cent_exp):
+    """Exact arg-max of bf16 keys and centroids whose squared norms underflow or overflow in fp32.  The centroids of a group
+    differ from each other by last places of every other channel, which the keys hardly weigh (2^-12 of the others): fp32
+    sums put up to two thirds of the keys on another one.  Eight-bit integers times powers of two, so that the sums are
+    exact in fp64 in any order."""
+    from longcontext_sqattn_paddle_b200.cache_hub import kmeans as km
+    g, t, k = 2, 700, 96
+    gen = torch.Generator().manual_seed(d)
+
+    def pick(lo, hi, *shape):
+        return torch.randint(lo, hi, shape, generator=gen).double() * (2.0 * torch.randint(0, 2, shape, generator=gen) - 1.0)
+
+    data, base = pick(128, 256, g, t, d), pick(130, 254, g, 1, d)
+    data[..., 1::2] *= 2.0 ** -12
+    bump = torch.zeros(g, k, d, dtype=torch.float64)
+    bump[..., 1::2] = torch.randint(-1, 2, (g, k, d // 2), generator=gen).double()
+    data, cent = (data * 2.0 ** key_exp).bfloat16(), ((base + bump) * 2.0 ** cent_exp).bfloat16()
+    score = data.double() @ cent.double().transpose(1, 2)
+    want = torch.where(score == score.amax(-1, keepdim=True), torch.arange(k), k).amin(-1)
+    _, idx, _ = km.k_means_train(data.cuda(), cent.cuda(), True)
+    assert torch.equal(idx.cpu().long(), want)
