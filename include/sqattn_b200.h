@@ -235,7 +235,7 @@ int sqattn_decode_merge(const float* partial_o, const float* partial_lse, int32_
 
 /* ---- kmeans (cache_hub/kmeans.py) --------------------------------------------------------- */
 
-/* Scratch of sqattn_kmeans_assign and sqattn_kmeans_index_add (flagged-token list, member lists), 256-byte aligned. */
+/* Scratch of sqattn_kmeans_assign, _index_add and _reverse_index (flagged tokens, member lists, counters), 256-byte aligned. */
 size_t sqattn_kmeans_workspace_bytes(int32_t groups, int32_t num_tokens, int32_t num_centroids);
 /* _triton_assign_kernel, kmeans.py:7-79: idx[g,t] = argmax_c <data[g,t], centroids[g,c]> (lowest c on
  * ties, exact: the fp32 tensor-core scores decide except for near ties, which are re-evaluated in fp64); when sums

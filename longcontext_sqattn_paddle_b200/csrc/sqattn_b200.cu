@@ -446,10 +446,10 @@ int launch_decode(const sqattn_decode_args* a, const DecodePlan& pl, cudaStream_
 
 // ---- kmeans helpers ----------------------------------------------------------------------------------------
 // scratch of the clustering entry points: [max centroid norm per group | flagged count | flagged list | arrival
-// slot per token | offsets per cluster | member list per group | counts per cluster (index_add only) | cluster counts of
-// the token ranges (reverse_index only)]
+// slot per token | offsets per cluster | member list per group | counts per cluster (index_add only)].  reverse_index uses
+// all of it for the cluster counts of its token ranges.
 struct KmWorkspace {
-  float* max_cnorm2; int* flagged_count; int* flagged; int* slot; int* offsets; int* members; int* counts; int* range_hist;
+  float* max_cnorm2; int* flagged_count; int* flagged; int* slot; int* offsets; int* members; int* counts;
   int flagged_cap;
   size_t total;
 };
@@ -467,7 +467,6 @@ KmWorkspace km_workspace(void* base, int32_t groups, int32_t num_tokens, int32_t
   w.offsets = reinterpret_cast<int*>(take(gk * sizeof(int)));
   w.members = reinterpret_cast<int*>(take(gt * sizeof(int)));
   w.counts = reinterpret_cast<int*>(take(gk * sizeof(int)));
-  w.range_hist = reinterpret_cast<int*>(take(gk * kSortRanges * sizeof(int)));
   w.total = off;
   return w;
 }
@@ -853,19 +852,23 @@ int sqattn_kmeans_reverse_index(const int32_t* idx, int32_t groups, int32_t num_
   if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255))
     return fail(SQATTN_ERR_WORKSPACE, "workspace of %zu bytes (256-byte aligned) required", need);
   const KmWorkspace w = km_workspace(workspace, groups, num_tokens, num_centroids);
-  // a range is a multiple of 32 tokens, at least 256 of them
-  int per_range = ((num_tokens + kSortRanges - 1) / kSortRanges + 31) / 32 * 32;
+  // as many token ranges as their cluster counts fit (never below two: the scratch has two integers per cluster; 64 while
+  // there are 32 tokens to a cluster); a range is a multiple of 32 tokens, at least 256 of them
+  int* range_hist = static_cast<int*>(workspace);
+  const size_t fit = w.total / (static_cast<size_t>(groups) * num_centroids * sizeof(int));
+  const int most = fit < static_cast<size_t>(kSortRanges) ? static_cast<int>(fit) : kSortRanges;
+  int per_range = ((num_tokens + most - 1) / most + 31) / 32 * 32;
   if (per_range < 256) per_range = 256;
   const dim3 ranges(groups, (num_tokens + per_range - 1) / per_range);   // any number of groups
   const int smem = (num_centroids < kSortClusters ? num_centroids : kSortClusters) * static_cast<int>(sizeof(int));
   SQ_CUDA(cudaFuncSetAttribute(kmeans_range_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   SQ_CUDA(cudaFuncSetAttribute(kmeans_range_emit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   for (int c0 = 0; c0 < num_centroids; c0 += kSortClusters)
-    kmeans_range_count_kernel<<<ranges, 32, smem, stream>>>(idx, w.range_hist, num_tokens, num_centroids, per_range, c0,
+    kmeans_range_count_kernel<<<ranges, 32, smem, stream>>>(idx, range_hist, num_tokens, num_centroids, per_range, c0,
                                                             num_centroids - c0 < kSortClusters ? num_centroids - c0 : kSortClusters);
-  kmeans_range_scan_kernel<<<dim3(groups, (num_centroids + 255) / 256), 256, 0, stream>>>(w.range_hist, cluster_size, ranges.y, num_centroids);
+  kmeans_range_scan_kernel<<<dim3(groups, (num_centroids + 255) / 256), 256, 0, stream>>>(range_hist, cluster_size, ranges.y, num_centroids);
   for (int c0 = 0; c0 < num_centroids; c0 += kSortClusters)
-    kmeans_range_emit_kernel<<<ranges, 32, smem, stream>>>(idx, w.range_hist, clusters, num_tokens, num_centroids, per_range, max_cluster_size, c0,
+    kmeans_range_emit_kernel<<<ranges, 32, smem, stream>>>(idx, range_hist, clusters, num_tokens, num_centroids, per_range, max_cluster_size, c0,
                                                            num_centroids - c0 < kSortClusters ? num_centroids - c0 : kSortClusters);
   SQ_CUDA(cudaGetLastError());
   return SQATTN_OK;

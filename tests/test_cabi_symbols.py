@@ -63,3 +63,12 @@ def test_centred_decode_is_planned_for_one_cta_per_sm(batch, n, hq, hkv):
     a.batch, a.num_q_heads, a.num_kv_heads, a.head_dim, a.kv_len, a.dtype = batch, hq, hkv, d, n, L.BF16
     items = L.lib.sqattn_decode_centered_workspace_bytes(C.byref(a)) // (4 * (hq * d + hq + hkv * d))   # padding is below one item
     assert 0.75 * min(148, hkv * batch * -(-n // 256)) <= items * hkv <= 148
+
+
+@pytest.mark.parametrize("g,t,k", [(8, 65536, 1024), (8, 4000, 64), (1, 300, 32), (8, 60000, 49152)])
+def test_clustering_scratch_holds_no_counters_of_its_own_for_the_sorted_lists(g, t, k):
+    """Norms, the flagged list, slots, members and two integers per cluster: the counters of the counting sort share them."""
+    from longcontext_sqattn_paddle_b200 import _lib as L
+    flagged = max(g * t // 16, 4096)
+    parts = [g, 1, flagged, g * t, g * k, g * t, g * k]
+    assert L.lib.sqattn_kmeans_workspace_bytes(g, t, k) == sum(-(-4 * n // 256) * 256 for n in parts)

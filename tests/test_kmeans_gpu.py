@@ -185,3 +185,16 @@ def test_assignment_where_fp32_has_no_squares_of_the_norms(d, key_exp, cent_exp)
     want = torch.where(score == score.amax(-1, keepdim=True), torch.arange(k), k).amin(-1)
     _, idx, _ = km.k_means_train(data.cuda(), cent.cuda(), True)
     assert torch.equal(idx.cpu().long(), want)
+
+
+@pytest.mark.parametrize("g,t,k", [(2, 700, 1024), (1, 5000, 9600), (3, 20000, 4992)])
+def test_member_lists_with_fewer_ranges_than_usual(g, t, k):
+    """Clusters of few tokens: the counters of the sort's token ranges fit only a few times into the scratch."""
+    from longcontext_sqattn_paddle_b200.cache_hub import kmeans as km
+    idx = torch.randint(0, k, (g, t), generator=torch.Generator().manual_seed(k), dtype=torch.int32)
+    n = torch.stack([torch.bincount(r.long(), minlength=k) for r in idx])
+    lists, size = (r.cpu().long() for r in km.reverse_index(idx.cuda(), k, int(n.max())))
+    assert torch.equal(size, n)
+    for b in range(g):
+        order = torch.sort(idx[b].long(), stable=True).indices          # members one cluster after another, in token order
+        assert torch.equal(lists[b][torch.arange(lists.shape[2]) < n[b][:, None]], order)
