@@ -6,8 +6,11 @@
 // tokens x 200 bins (this one 1.10 ms); the products of one sweep are 0.15 ms of the measured tensor rate, its exponentials 0.2 ms of the
 // special-function units.  Hence:
 //   * a thread owns one query row (a TMEM lane) and meets its keys in order, so its bins never increase: a bin is one
-//     run, kept as A0 = sum a and A1 = sum a * (j - ref) with a = 2^(score - base) NOT normalised, and stored once, in a
-//     per-row histogram in shared memory; the row sum is known at the end and scales the stored bins then.  base is the
+//     run, kept as A0 = sum a and A1 = sum a * (ref - j) with a = 2^(score - base) NOT normalised, and stored once, in a
+//     per-row histogram in shared memory; the row sum is known at the end and scales the stored bins then.  ref is the last
+//     visible key met so far: the run's weighted sum A0 * w(ref) + A1 * (bins per key) has no negative term, so nothing
+//     cancels however narrow the bins are (relative to the first key of a chunk, rows of 8 keys with 200 bins were off by
+//     2e-5).  base is the
 //     maximum of the row's first keys; fp32 holds a up to 2^60 above it, so it moves (and the stored bins are rescaled)
 //     only past that.
 //   * the bin of a key is not computed per pair: the run knows the first key of the next bin, from integer arithmetic
@@ -67,7 +70,7 @@ struct WindowRow {
   float* slot;               // where the current run goes when it ends: its bin of `hist`, or aside
   const uint8_t* tie;        // [nbins] see edge()
   float base;                // raw score that the weights are relative to; -inf: no key yet
-  float a0, a1, l;           // the current run (a1 relative to the current chunk's first key), sum of the finished runs
+  float a0, a1, l;           // the current run (a1 relative to the current chunk's last visible key), sum of the finished runs
   int cur, next, first;      // bin of the current run (-1: none yet), first key behind it, bin of the first run
   int eq, er;                // the current bin's lower edge, cur * ctx = eq * nbins + er keys away
   int dq, dr;                // ctx = dq * nbins + dr: one bin
@@ -110,8 +113,8 @@ struct WindowRow {
     slot = hist + cur * 128;
     edge();
   }
-  __device__ __forceinline__ void flush(float t0) {   // t0 = weight per unit at the key that a1 is relative to
-    *slot = __fmaf_rn(a0, t0, -cinv * a1);
+  __device__ __forceinline__ void flush(float t0) {   // t0 = weight at the key that a1 is relative to
+    *slot = __fmaf_rn(a0, t0, cinv * a1);
     l += a0;
   }
   __device__ __forceinline__ float weight(int j) const { return __fmaf_rn(static_cast<float>(i - j), cinv, 1.0f); }
@@ -139,7 +142,8 @@ struct WindowRow {
     for (int c = 3; c < 31; c += 2) mx = max3(mx, __uint_as_float(r[c]), __uint_as_float(r[c + 1]));
     look_at_max(fmaxf(mx, __uint_as_float(r[31])));
     if (cur < 0) begin(c0);
-    const float sh = shift(), t0 = weight(c0);
+    const float sh = shift(), t0 = weight(c0 + 31);
+    a1 = __fmaf_rn(32.0f, a0, a1);
     float x[32];
 #pragma unroll
     for (int c = 0; c < 32; ++c) x[c] = ex2_approx(__fmaf_rn(__uint_as_float(r[c]), c2, sh));
@@ -149,8 +153,8 @@ struct WindowRow {
       float v0 = 0.f, v1 = 0.f;
 #pragma unroll
       for (int c = s; c < s + kSub; ++c) {
-        if (c < nb) { a0 += x[c]; a1 = __fmaf_rn(x[c], static_cast<float>(c), a1); }
-        else { v0 += x[c]; v1 = __fmaf_rn(x[c], static_cast<float>(c), v1); }
+        if (c < nb) { a0 += x[c]; a1 = __fmaf_rn(x[c], static_cast<float>(31 - c), a1); }
+        else { v0 += x[c]; v1 = __fmaf_rn(x[c], static_cast<float>(31 - c), v1); }
       }
       if (nb < s + kSub) {
         flush(t0);
@@ -158,7 +162,6 @@ struct WindowRow {
         lower();
       }
     }
-    a1 = __fmaf_rn(-32.0f, a0, a1);
   }
   // 8 keys from c0 on, any of them past the row or in the sink, bins of any width
   __device__ __forceinline__ void chunk8(const uint32_t (&r)[8], int c0) {
@@ -167,7 +170,9 @@ struct WindowRow {
 #pragma unroll
     for (int e = 1; e < 8; ++e) mx = (c0 + e <= i) ? fmaxf(mx, __uint_as_float(r[e])) : mx;
     look_at_max(mx);
-    const float sh = shift(), t0 = weight(c0);
+    const int last = min(7, i - c0);
+    const float sh = shift(), t0 = weight(c0 + last), to_last = static_cast<float>(last);
+    a1 = __fmaf_rn(to_last + 1.0f, a0, a1);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int j = c0 + e;
@@ -189,10 +194,9 @@ struct WindowRow {
           begin(j);
         }
         a0 += x;
-        a1 = __fmaf_rn(x, static_cast<float>(e), a1);
+        a1 = __fmaf_rn(x, to_last - static_cast<float>(e), a1);
       }
     }
-    a1 = __fmaf_rn(-8.0f, a0, a1);
   }
 };
 
@@ -316,7 +320,7 @@ window_hist_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     // bins of 9 (17) keys and more: their edges are at least 8 (16) keys apart, rounded or not
     const bool wide = i_first + 31 < p.n && i_first - p.sink >= 9 * p.nbins, very_wide = wide && i_first - p.sink >= 17 * p.nbins;
     bool ok = true;
-    int ref = 0;                                                        // key that a1 is relative to
+    int ref = 0;                                                        // first key not met yet
     const int tile0 = part_begin(g), tiles = part_begin(g + 1) - tile0;
     for (int u = 0; u < tiles; ++u) {
       const uint32_t slot = 2 * g + (u & 1);
@@ -347,8 +351,8 @@ window_hist_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       tc_fence_before();
       mbar_arrive(bar_s_empty + 8 * slot);
     }
-    // the row's last run: a1 is relative to the key behind the last chunk that was not skipped
-    if (w.cur >= 0) w.flush(w.weight(min(ref, (w.i & ~7) + 8)));
+    // the row's last run: a1 is relative to the last visible key of the part
+    if (w.cur >= 0) w.flush(w.weight(min(ref - 1, w.i)));
     row_l = w.l; row_base = w.base;
     fac_s[g * 128 + row] = w.base;
     first_s[g * 128 + row] = w.first;

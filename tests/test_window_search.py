@@ -67,3 +67,18 @@ def test_relative_histogram_at_tile_and_bin_edges(n, d, bins, sink):
         a = wo.attention_map(q, k)
         for h in range(4):
             np.testing.assert_allclose(hist[h], wo.relative_histogram_with_sink(a[h], bins, sink), rtol=5e-5, atol=1e-30)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,bins", [(8, 200), (40, 248), (200, 200), (1000, 200), (3000, 100)])
+def test_relative_histogram_keeps_fp32_precision_in_bins_narrower_than_a_key(n, bins):
+    """Without a sink, rows of a few keys have all their weight in bins much narrower than a key.  All terms of a bin are
+    positive, so its relative error is a pair's: 2^-22 of the exponential, 2^-23 * 10 * 4 / 8 = 6e-7 of an fp32 score of
+    magnitude <= 10 summed over 64 products, and 1e-6 for some sixteen roundings of sums, weight and normalisation."""
+    from longcontext_sqattn_paddle_b200.sqattn import window_search as ws
+    g = torch.Generator().manual_seed(n)
+    q, k = ((torch.randn(h, n, 64, generator=g) * 0.5).to(torch.bfloat16) for h in (4, 2))
+    hist = ws.attention_histograms(q.cuda(), k.cuda(), relative=True, num_bins=bins, sink_len=0).cpu().numpy()
+    a = wo.attention_map(q, k)
+    for h in range(4):
+        np.testing.assert_allclose(hist[h], wo.relative_histogram_with_sink(a[h], bins, 0), rtol=2e-6, atol=1e-30)
