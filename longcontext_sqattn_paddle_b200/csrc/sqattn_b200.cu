@@ -1019,6 +1019,8 @@ int sqattn_window_histogram(const void* q, const void* k, int32_t dtype, int32_t
   if (head_dim % 8 || head_dim <= 0 || head_dim > 256) return fail(SQATTN_ERR_UNSUPPORTED, "head_dim %d", head_dim);
   if (num_q_heads <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads || seq_len <= 0 || num_bins <= 0 || sink < 0)
     return fail(SQATTN_ERR_INVALID_ARG, "bad sizes");
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k)) & 15)
+    return fail(SQATTN_ERR_INVALID_ARG, "q and k need 16-byte alignment");   // every kernel below reads 16 bytes at a time
   WindowHistParams p;
   p.q = static_cast<const uint8_t*>(q); p.k = static_cast<const uint8_t*>(k); p.hist = hist;
   p.hq = num_q_heads; p.groups = num_q_heads / num_kv_heads; p.n = seq_len; p.d = head_dim; p.nbins = num_bins;
@@ -1027,7 +1029,7 @@ int sqattn_window_histogram(const void* q, const void* k, int32_t dtype, int32_t
   // Relative distances go to the tcgen05 kernel while the rows' histograms fit into shared memory and a bin is no finer
   // than its edge arithmetic assumes.  Absolute distances have a bin per key, which that kernel's runs gain nothing from.
   if ((head_dim == 64 || head_dim == 128) && relative && num_bins <= kWtMaxBins &&
-      seq_len <= static_cast<long long>(kWtKeysPerBin) * num_bins && !((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k)) & 15) &&
+      seq_len <= static_cast<long long>(kWtKeysPerBin) * num_bins &&
       static_cast<long long>((seq_len + kWtRows - 1) / kWtRows) * num_q_heads <= 0x7fffffffll)
     return head_dim == 128 ? launch_window_hist_tc<128>(p, dtype, stream) : launch_window_hist_tc<64>(p, dtype, stream);
   if (head_dim == 64 || head_dim == 128) {

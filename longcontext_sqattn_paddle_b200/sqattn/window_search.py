@@ -18,11 +18,12 @@ def attention_histograms(q: torch.Tensor, k: torch.Tensor, *, relative: bool, nu
                          out: torch.Tensor = None) -> torch.Tensor:
     """q [Hq,N,D], k [Hkv,N,D] (CUDA, 16-bit) -> fp64 [Hq, num_bins]; ``out`` accumulates over samples."""
     _require_cuda(q, k)
+    q, k = (t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format) for t in (q, k))
     hq, n, d = q.shape
     if out is None:
         out = torch.zeros(hq, num_bins, dtype=torch.float64, device=q.device)
-    L.check(L.lib.sqattn_window_histogram(q.contiguous().data_ptr(), k.contiguous().data_ptr(), _dt(q.dtype), hq,
-                                          k.shape[0], n, d, int(relative), num_bins, sink_len, out.data_ptr(), _stream()))
+    L.check(L.lib.sqattn_window_histogram(q.data_ptr(), k.data_ptr(), _dt(q.dtype), hq, k.shape[0], n, d, int(relative),
+                                          num_bins, sink_len, out.data_ptr(), _stream()))
     return out
 
 

@@ -82,3 +82,29 @@ def test_relative_histogram_keeps_fp32_precision_in_bins_narrower_than_a_key(n, 
     a = wo.attention_map(q, k)
     for h in range(4):
         np.testing.assert_allclose(hist[h], wo.relative_histogram_with_sink(a[h], bins, 0), rtol=2e-6, atol=1e-30)
+
+
+def test_unaligned_inputs_are_refused_before_a_kernel_reads_them():
+    from longcontext_sqattn_paddle_b200 import _lib as L
+    for q, k in ((0x1008, 0x2000), (0x1000, 0x2002)):
+        for d in (32, 64, 128):
+            assert L.lib.sqattn_window_histogram(q, k, L.BF16, 4, 2, 100, d, 1, 50, 0, 0x3000, None) == L.ERR_INVALID_ARG
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("relative", [True, False])
+def test_histograms_of_views(relative):
+    """Token-major views of both inputs (each has to be copied, and the copies have to live together), and unaligned ones."""
+    from longcontext_sqattn_paddle_b200.sqattn import window_search as ws
+    n, d, bins = 900, 64, 100
+    g = torch.Generator(device="cuda").manual_seed(7)
+    q, k = (torch.randn(h, n, d, generator=g, device="cuda").to(torch.bfloat16) for h in (4, 2))
+
+    def hist(a, b):
+        return ws.attention_histograms(a, b, relative=relative, num_bins=bins if relative else n, sink_len=64).cpu().numpy()
+
+    want = hist(q, k)
+    token_major = [t.transpose(0, 1).contiguous().transpose(0, 1) for t in (q, k)]
+    shifted = [torch.cat([t.new_zeros(3), t.flatten()])[3:].view(t.shape) for t in (q, k)]
+    for a, b in (token_major, shifted):
+        np.testing.assert_allclose(hist(a, b), want, rtol=1e-5)        # the same values, a block's fp32 sums in another order
