@@ -108,3 +108,26 @@ def test_histograms_of_views(relative):
     shifted = [torch.cat([t.new_zeros(3), t.flatten()])[3:].view(t.shape) for t in (q, k)]
     for a, b in (token_major, shifted):
         np.testing.assert_allclose(hist(a, b), want, rtol=1e-5)        # the same values, a block's fp32 sums in another order
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,bins,sink", [(33001, 200, 0), (40000, 96, 256), (65001, 100, 0)])
+def test_relative_histogram_of_rows_beyond_31250_keys(n, bins, sink):
+    """There the reference's fp32 expression can put the key beside a bin's edge on either side, and the kernel asks the
+    expression itself.  The definition in fp64 on the GPU, bins in fp32 as the reference has them; the bar is that of
+    test_relative_histogram_at_tile_and_bin_edges (one key on the wrong side of an edge moves a bin by 1 / keys per bin)."""
+    from longcontext_sqattn_paddle_b200.sqattn import window_search as ws
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, k = (torch.randn(1, n, 64, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    hist = ws.attention_histograms(q, k, relative=True, num_bins=bins, sink_len=sink)
+    ref = torch.zeros(bins, dtype=torch.float64, device="cuda")
+    cols, kt = torch.arange(n, device="cuda")[None], k[0].double().T
+    for r in range(0, n, 512):
+        rows = torch.arange(r, min(r + 512, n), device="cuda")[:, None]
+        a = torch.softmax((q[0, r:r + 512].double() @ kt / 8.0).masked_fill(cols > rows, float("-inf")), -1)
+        rel = (rows - cols).float() / torch.clamp(rows.float() - sink, min=1)
+        rel[rows.squeeze(1) <= sink] = 0
+        b = torch.clamp((rel * bins).floor().long(), 0, bins - 1)
+        w = (a * (rel * bins + 1)).masked_fill((cols > rows) | (cols < sink), 0.0)
+        ref += torch.zeros(len(rows), bins, dtype=torch.float64, device="cuda").scatter_add_(1, b, w).sum(0)
+    np.testing.assert_allclose(hist[0].cpu().numpy(), ref.cpu().numpy(), rtol=5e-5)
