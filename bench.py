@@ -769,13 +769,13 @@ def run_kernel_only(args):
         fn = lambda: km.k_means_train(keys, cent, True)
         work, unit = 2.0 * g8 * n * kc * D / 1e12, "TFLOP/s"
     elif args.kernel_only == "window":
-        # the blockwise attention-energy histogram of one layer (28 heads) at --seq tokens: 2*D flops per causal pair
+        # the attention-energy histogram of one layer (28 heads) at --seq tokens, one sweep: 2*D flops per causal pair
         from longcontext_sqattn_paddle_b200.sqattn import window_search as ws
         g = torch.Generator(device=dev).manual_seed(4)
         qw = torch.randn(HQ, n, D, device=dev, dtype=torch.bfloat16, generator=g)
         kw = torch.randn(HKV, n, D, device=dev, dtype=torch.bfloat16, generator=g)
         fn = lambda: ws.attention_histograms(qw, kw, relative=True, num_bins=200, sink_len=SINK)
-        work, unit = 2.0 * 2 * D * HQ * (n * (n + 1) / 2) / 1e12, "TFLOP/s"    # two sweeps (maximum / sum, then weights)
+        work, unit = 2.0 * D * HQ * (n * (n + 1) / 2) / 1e12, "TFLOP/s"
     elif args.kernel_only == "retrieval":
         # select + gather + ragged decode for 4 clustered sequences of --seq tokens, 4096-token budget
         from longcontext_sqattn_paddle_b200.cache_hub import ClusteredKV, RaggedClusteredDecoder

@@ -2,16 +2,15 @@
 // kernel): scores <k_t, x_c> for 256 tokens x all centroids of a group per CTA as tcgen05 MMAs with the
 // accumulators in tensor memory, and a running top-2 per token in the epilogue.
 //
-//   warp 0        TMA producer: the CTA's two 128-token tiles once, then 256-centroid tiles into a 2-stage ring
+//   warp 0        TMA producer: an item's two 128-token tiles, then its group's 256-centroid tiles into a 2-stage ring
 //   warp 1        MMA issuer: for every centroid tile, S_a = tokens_a x centroids^T (M128 N256 K16 x D/16) for the
 //                 two token tiles a = 0, 1 in turn; owns the 512 TMEM columns (two 256-column accumulators)
 //   warps 2..5    epilogue of token tile 0, warps 6..9 of token tile 1: one token per thread (a TMEM lane)
-// While the epilogue warps of one token tile scan their 256 scores, the tensor core computes the other tile's, so
-// the two never wait for each other as long as a scan (about 3 instructions per score) is shorter than a tile's
-// 1024 tensor-pipe clocks.  Every centroid tile staged in shared memory is used by both token tiles, which halves
-// the L2 traffic per flop.  A CTA (one per SM) walks several 256-token items: with one item per CTA the start-up of
-// each (tensor memory, barriers, the first tiles) lay open: 268 us an assignment of 8 x 65536 keys to 1024 centroids, 220
-// now.  The scan's minima and maxima run at half rate, 107 us of it if nothing else stood in the way.
+// While the epilogue warps of one token tile scan their 256 scores, the tensor core computes the other tile's.  The scan
+// bounds it: 5.8 instructions per score (its minima and maxima at half rate) behind the tensor-memory loads, 220 us for
+// 8 x 65536 keys and 1024 centroids whose products take 84 us of the measured rate.  Every centroid tile staged in shared
+// memory is used by both token tiles, which halves the L2 traffic per flop.  A CTA (one per SM) walks several 256-token
+// items: with one item per CTA the start-up of each (tensor memory, barriers, the first tiles) lay open (268 us).
 //
 // Exactness: the fp32 tensor-core score is not the exact inner product, so a token whose best and second-best
 // scores are closer than a bound on that error is put on a list and re-scored in fp64 by kmeans_recheck_list_kernel
@@ -36,7 +35,6 @@ constexpr float kKtTol = 1.25e-4f;
 constexpr float kKtMinNorm2 = 7.888609e-31f;
 
 struct KmeansTcParams {
-  const uint8_t* data;      // [G, T, D] for the token norms
   int* idx;                 // [G, T]
   int* flagged;             // [cap] packed g * T + t of tokens to re-score
   int* flagged_count;       // number of entries (may exceed cap: the overflow is re-scored by a full sweep)

@@ -478,9 +478,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
         // more than kLazyLog2 (so P <= 2^kLazyLog2): O then needs its rescale (a wait for the previous P V plus a
         // TMEM round trip) a few times per row instead of whenever the maximum moves.  Steps whose P is rounded
         // through e4m3 keep base == running maximum: p <= 1 as the rounding rule expects, and P is f16(e4m3(448 p) / 448)
-        // itself.  (A lazy base there has to bring P to it by the factor 2^(m - base), which is no power of two: 8192
-        // tokens took 27 us less, but the f16 rounding of the scaled P lost the exact P = 1 of the row's maximum and was
-        // a tenth larger on average.)
+        // itself.  (A lazy base there has to bring P to it by the factor 2^(m - base), which is no power of two: the
+        // operator at 8192 tokens took 262 us instead of 311, but the f16 rounding of the scaled P lost the exact P = 1 of
+        // the row's maximum and was a tenth larger on average.)
         if (m_new > base + (fp8 ? 0.0f : kLazyLog2)) {
           alpha = ex2_approx(base - m_new);
           base = m_new;

@@ -114,14 +114,13 @@ __global__ void kmean_partial_kernel(View4 k, float* partial) {
   extern __shared__ float red[];
   kmean_partial_body<BF16>(k, partial, blockIdx.y, blockIdx.x, red);
 }
-// mean[bh][d] = (sum of the partials in chunk order) / n; n == 0 stores the plain column sums (the
-// sequence-parallel path all-reduces the sums of the shards before dividing)
-__global__ void kmean_final_kernel(const float* partial, float* mean, int d, int n) {
+// sums[bh][d] = the partials in chunk order (the sequence-parallel path all-reduces the sums of the shards)
+__global__ void kmean_final_kernel(const float* partial, float* sums, int d) {
   const int bh = blockIdx.x;
   if (threadIdx.x < d) {
     float s = 0.f;
     for (int c = 0; c < kMeanChunks; ++c) s += partial[(static_cast<long long>(bh) * kMeanChunks + c) * d + threadIdx.x];
-    mean[bh * d + threadIdx.x] = n > 0 ? s / static_cast<float>(n) : s;
+    sums[bh * d + threadIdx.x] = s;
   }
 }
 
@@ -165,11 +164,6 @@ __device__ __forceinline__ float fake_quant_value(float x, float absmax, int qty
   return s * scale;
 }
 
-// Integer grid, fast path for 8 values: q = x * (1/scale) is within 2e-5 of the exact quotient
-// x / scale (|q| <= qmax * (1 + 2^-22), so the clamp of the reference never acts), hence unless q lies within
-// 1e-4 of a half-integer its nearest integer IS round(x / scale) in either rounding mode; a group with such a
-// value (rare) is redone with exact divisions.  Results are identical to fake_quant_value(..., INT, ...).
-
 // rintf of two values below 2^22 in magnitude: adding and taking off 1.5 * 2^23 leaves the nearest integer (ties to even),
 // the sign goes back on for the negative zeros.  The conversion unit's own rounding runs at an eighth of this rate.
 __device__ __forceinline__ uint64_t rint2_small(uint64_t x2) {
@@ -182,7 +176,10 @@ __device__ __forceinline__ uint64_t rint2_small(uint64_t x2) {
 
 // The integer grid for the 8 values a thread holds of one row, on packed fp32 pairs, returning the 8 results
 // rounded to the 16-bit type (and, for queries, multiplied by q_scale and rounded again) as four packed words.
-// Every operation is the IEEE round-to-nearest one of the scalar path above, so the bits are the same.
+// q = x * (1/scale) is within 2e-5 of the exact quotient x / scale (|q| <= qmax * (1 + 2^-22), so the clamp of the
+// reference never acts), hence unless q lies within 1e-4 of a half-integer its nearest integer IS round(x / scale) in
+// either rounding mode; a group with such a value (rare) is redone with exact divisions.  The bits are those of
+// fake_quant_value(..., INT, ...).
 template <bool BF16, bool kScale>
 __device__ __forceinline__ uint4 fake_quant_int_row8(const float (&x)[8], float absmax, float qmax, int half_even, float q_scale) {
   const float scale = __fdiv_rn(absmax, qmax), inv = __fdiv_rn(1.0f, scale);

@@ -31,7 +31,7 @@ double sm_scale_log2(int head_dim, int head_dim_og = 0) {
 // Which kernels get it is a measured choice (1M-token decode sharded over 2 GPUs, 28 layers per step, graph replay):
 // none 4.806 ms, the merge kernels only 4.800 ms, merge and decode kernels 5.245 ms (a decode grid that becomes
 // resident behind the running one slows it down), so of those only the merges do by default.  The operator's preparation
-// and its attention kernel do: 8192 tokens, FP8 P: 280 us a call with, 293 without.
+// and its attention kernel do: 8192 tokens, FP8 P: 310 us a call with, 320 without; 1000 tokens: 46.8 and 48.3.
 // SQATTN_B200_OVERLAP (read once) overrides with a bit mask of kernel classes: 1 = merge kernels, 2 = decode kernel,
 // 4 = preparation and prefill kernels.
 int overlap_mask() {
@@ -261,10 +261,14 @@ struct DecodePlan {
 // leave more ends) lets the short items and the second halves fill up the memory system instead.  In a graph, before and
 // after: 8 sequences of 2000..65536 keys, 32/8 heads 122 and 112 us, 28/4 heads 69.6 and 62.4; 5 of 10000..40000 87 and
 // 79; 3 of 20000 52 and 48.5; beyond two CTAs per SM a second wave costs more than it evens out (121, 77, 96, 60).
+// Between one and a half and two, up to eight sequences lose or draw (62.4 and 63.5; 78.8 and 79.3; 3 of 100000..300000 178
+// and 185), more of them gain: 16 of 1000..30000, 32/8 heads 117 and 101; 10 of 20000 141 and 130; 24 of 1000..30000, 28/4
+// heads 87.6 and 82.4; 16 of 20000 111.8 and 111.2; 9 of 30000 lose, 92.9 and 94.8.
 // Keys through an index list: two per SM as well, since the warps' own chain per tile bounds the kernel there (64 lists
 // of 4096 keys, FP8 P: 51 and 36 us; 56: 43 and 30; 16: 20 and 17).
 // The kernel that also adds up columns (centred) has 320 threads of more than 150 registers, so one CTA fits on an SM and
-// anything beyond 148 CTAs is a second wave.
+// anything beyond 148 CTAs is a second wave: 2 x 32000 keys, 4 KV heads 46.1 us with the plan of the plain kernel, 34.7 with
+// at most 148 CTAs; 2 x 100000 101.9 and 79.1; 1 x 32000 with 8 KV heads (152 CTAs otherwise) 47.2 and 33.7.
 int plan_decode(const sqattn_decode_args* a, DecodePlan* pl, bool centered = false) {
   if (!a) return fail(SQATTN_ERR_INVALID_ARG, "args is null");
   if (a->head_dim != 64 && a->head_dim != 128) return fail(SQATTN_ERR_UNSUPPORTED, "head_dim %d: only 64 and 128", a->head_dim);
@@ -496,7 +500,7 @@ int km_launch_assign(const void* data, const void* centroids, int32_t dtype, int
   if ((rc = make_tmap_bhnd(&td, data, dtype, sd * groups, sd, D, 1, groups, num_tokens, D, 128, "kmeans data"))) return rc;
   if ((rc = make_tmap_bhnd(&tc, centroids, dtype, sc * groups, sc, D, 1, groups, num_centroids, D, kKtCent, "kmeans centroids"))) return rc;
   KmeansTcParams p;
-  p.data = static_cast<const uint8_t*>(data); p.idx = idx; p.flagged = w.flagged; p.flagged_count = w.flagged_count;
+  p.idx = idx; p.flagged = w.flagged; p.flagged_count = w.flagged_count;
   p.flagged_cap = w.flagged_cap; p.max_cnorm2 = w.max_cnorm2; p.groups = groups; p.num_tokens = num_tokens; p.num_centroids = num_centroids;
   p.bf16 = dtype == SQATTN_BF16;
   using L = KmeansTcSmem<D>;
@@ -574,7 +578,7 @@ int sqattn_debug_prefill_timeline(const sqattn_prefill_args* args, float* dump, 
 
 size_t sqattn_prep_workspace_bytes(const sqattn_prep_args* a) {
   if (!a) return 0;
-  return static_cast<size_t>(a->batch) * a->num_kv_heads * (kMeanChunks + 1) * a->head_dim * sizeof(float);
+  return static_cast<size_t>(a->batch) * a->num_kv_heads * kMeanChunks * a->head_dim * sizeof(float);
 }
 
 int sqattn_prep_qkv(const sqattn_prep_args* a, sqattn_stream_t stream_) {
@@ -643,7 +647,7 @@ int sqattn_k_column_sums(const sqattn_tensor* k, int32_t batch, int32_t num_kv_h
   float* partial = static_cast<float*>(workspace);
   if (dtype == SQATTN_BF16) kmean_partial_kernel<true><<<mg, 256, lanes * head_dim * sizeof(float), stream>>>(kk, partial);
   else kmean_partial_kernel<false><<<mg, 256, lanes * head_dim * sizeof(float), stream>>>(kk, partial);
-  kmean_final_kernel<<<batch * num_kv_heads, 128, 0, stream>>>(partial, sums, head_dim, 0);
+  kmean_final_kernel<<<batch * num_kv_heads, 128, 0, stream>>>(partial, sums, head_dim);
   SQ_CUDA(cudaGetLastError());
   return SQATTN_OK;
 }

@@ -3,7 +3,7 @@
 //
 // What bounds it: one exponential per (query, key) pair.  The mma.sync kernel swept the keys twice (statistics, then
 // normalised weights), computed two exponentials and an IEEE division per pair and took 10.6 ms for 28 heads x 8192
-// tokens x 200 bins (this one 1.10 ms); the products of one sweep are 0.15 ms of the measured tensor rate, its exponentials 0.2 ms of the
+// tokens x 200 bins (this one 1.11 ms); the products of one sweep are 0.15 ms of the measured tensor rate, its exponentials 0.2 ms of the
 // special-function units.  Hence:
 //   * a thread owns one query row (a TMEM lane) and meets its keys in order, so its bins never increase: a bin is one
 //     run, kept as A0 = sum a and A1 = sum a * (ref - j) with a = 2^(score - base) NOT normalised, and stored once, in a

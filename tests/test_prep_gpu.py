@@ -132,9 +132,9 @@ def test_q_fake_quant_inside_the_attention_kernel_is_bit_identical(dtype, qtype)
 
 
 @pytest.mark.parametrize("n,hq,hkv,d", [(1, 4, 2, 128), (63, 4, 1, 64), (8257, 28, 4, 128), (20011, 32, 8, 128), (16500, 32, 8, 64)])
-def test_prep_rounds_of_rows(n, hq, hkv, d):
-    """Rows are independent given K's mean, so a call whose blocks go over several rounds of rows equals calls on short
-    slices, whose blocks take one, bit for bit; so do calls that prepare one tensor at a time."""
+def test_prep_of_slices_equals_the_whole(n, hq, hkv, d):
+    """Rows are independent given K's mean: a whole call, whose K blocks add the mean up themselves, equals calls on slices
+    that are given the mean, bit for bit (row blocks that end anywhere); so do calls that prepare one tensor at a time."""
     from longcontext_sqattn_paddle_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(n)
     qkv = torch.randn(1, n, (hq + 2 * hkv) * d, generator=g, device="cuda", dtype=torch.bfloat16)
