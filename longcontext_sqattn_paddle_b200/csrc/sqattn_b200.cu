@@ -266,7 +266,7 @@ struct DecodePlan {
 // heads 87.6 and 82.4; 16 of 20000 111.8 and 111.2; 9 of 30000 lose, 92.9 and 94.8.
 // Keys through an index list: two per SM as well, since the warps' own chain per tile bounds the kernel there (64 lists
 // of 4096 keys, FP8 P: 51 and 36 us; 56: 43 and 30; 16: 20 and 17).
-// The kernel that also adds up columns (centred) has 320 threads of more than 150 registers, so one CTA fits on an SM and
+// The kernel that also adds up columns (centred) has 320 threads of 104 to 166 registers, so one CTA fits on an SM and
 // anything beyond 148 CTAs is a second wave: 2 x 32000 keys, 4 KV heads 46.1 us with the plan of the plain kernel, 34.7 with
 // at most 148 CTAs; 2 x 100000 101.9 and 79.1; 1 x 32000 with 8 KV heads (152 CTAs otherwise) 47.2 and 33.7.
 int plan_decode(const sqattn_decode_args* a, DecodePlan* pl, bool centered = false) {
