@@ -10,9 +10,8 @@
 //     per-row histogram in shared memory; the row sum is known at the end and scales the stored bins then.  ref is the last
 //     visible key met so far: the run's weighted sum A0 * w(ref) + A1 * (bins per key) has no negative term, so nothing
 //     cancels however narrow the bins are (relative to the first key of a chunk, rows of 8 keys with 200 bins were off by
-//     2e-5).  base is the
-//     maximum of the row's first keys; fp32 holds a up to 2^60 above it, so it moves (and the stored bins are rescaled)
-//     only past that.
+//     4e-6, 3e-7 so).  base is the maximum of the row's first keys; fp32 holds a up to 2^60 above it, so it moves (and the
+//     stored bins are rescaled) only past that.
 //   * the bin of a key is not computed per pair: the run knows the first key of the next bin, from integer arithmetic
 //     that steps from one bin's edge to the next, and from how the reference's fp32 expression rounds where an edge is a
 //     whole number of keys (edge()).
