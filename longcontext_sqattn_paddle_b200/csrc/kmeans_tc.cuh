@@ -2,15 +2,19 @@
 // kernel): scores <k_t, x_c> for 256 tokens x all centroids of a group per CTA as tcgen05 MMAs with the
 // accumulators in tensor memory, and a running top-2 per token in the epilogue.
 //
-//   warp 0        TMA producer: an item's two 128-token tiles, then its group's 256-centroid tiles into a 2-stage ring
-//   warp 1        MMA issuer: for every centroid tile, S_a = tokens_a x centroids^T (M128 N256 K16 x D/16) for the
-//                 two token tiles a = 0, 1 in turn; owns the 512 TMEM columns (two 256-column accumulators)
+//   warp 0        TMA producer: an item's two 128-token tiles, two items deep, and its group's 128-centroid tiles into a
+//                 3-stage ring
+//   warp 1        MMA issuer: for every centroid tile, S_a = tokens_a x centroids^T (M128 N128 K16 x D/16) for the
+//                 two token tiles a = 0, 1 in turn; owns the 512 TMEM columns (two 128-column accumulators per token tile)
 //   warps 2..5    epilogue of token tile 0, warps 6..9 of token tile 1: one token per thread (a TMEM lane)
-// While the epilogue warps of one token tile scan their 256 scores, the tensor core computes the other tile's.  The scan
-// bounds it: 5.8 instructions per score (its minima and maxima at half rate) behind the tensor-memory loads, 220 us for
-// 8 x 65536 keys and 1024 centroids whose products take 84 us of the measured rate.  Every centroid tile staged in shared
-// memory is used by both token tiles, which halves the L2 traffic per flop.  A CTA (one per SM) walks several 256-token
-// items: with one item per CTA the start-up of each (tensor memory, barriers, the first tiles) lay open (268 us).
+// The epilogue warps scan one accumulator while the tensor core fills the other; every centroid tile staged in shared memory
+// is used by both token tiles, which halves the L2 traffic per flop.  The scan bounds it: five minima and maxima per two
+// scores on a pipe that takes one in two clocks.  A score's column is put into it on the FMA pipe, which is otherwise idle:
+// scaled to +-500000 and rounded to a whole number by adding 1.5 * 2^23, then the column added as 32nds (6.2 clocks per score
+// and scheduler; with the column in the low bits by (bits & ~31) | column, two logic operations on the pipe of the minima, 9.5).
+// 8 x 65536 keys, 1024 centroids: 215 us with the logic operations, 179 with one of them (LOP3), 165 like this, 109 with the
+// scan left out, and 84 at the measured matrix rate.  A CTA (one per SM) walks several 256-token items: with one item per CTA
+// the start-up of each (tensor memory, barriers, the first tiles) lay open (268 us).
 //
 // Exactness: the fp32 tensor-core score is not the exact inner product, so a token whose best and second-best
 // scores are closer than a bound on that error is put on a list and re-scored in fp64 by kmeans_recheck_list_kernel
@@ -25,11 +29,16 @@
 namespace sq {
 
 constexpr int kKtTokens = 256;    // tokens per CTA (two M = 128 tiles)
-constexpr int kKtCent = 256;      // centroids per MMA group (N)
-constexpr int kKtStages = 2;
+constexpr int kKtCent = 128;      // centroids per MMA group (N)
+constexpr int kKtStages = 3;
 // |tensor-core fp32 sum - exact| is bounded by (terms * 2^-22) * sum|terms| <= 2^-15 |k||x| for 128 terms; the two
 // scores that are compared each carry it, and the factor of two on top covers an accumulator that truncates
 constexpr float kKtTol = 1.25e-4f;
+// The scan compares scores in units of |k| max|x| / kKtScale, rounded to whole ones (below 2^19, so that 32nds beside them are
+// exact).  Two scores that are kKtTol |k| max|x| apart differ by kKtTol * kKtScale = 62.5 there, less two roundings of a half
+// and 31/32 of column; the rest covers the rounding of the scale itself.
+constexpr float kKtScale = 500000.0f;
+constexpr float kKtGap = 64.6f;
 // Squared norms from here on (2^-100) bound the error as stated: squares and products that underflow are below 2^-126 each,
 // less than 2^-119 in all, where the bound is at least 1.25e-4 * 2^-100 = 2^-113.
 constexpr float kKtMinNorm2 = 7.888609e-31f;
@@ -48,10 +57,10 @@ struct KmeansTcSmem {
   static constexpr int kABytes = 128 * D * 2;
   static constexpr int kBBytes = kKtCent * D * 2;
   static constexpr int kAOff = 0;
-  static constexpr int kBOff = 2 * kABytes;
+  static constexpr int kBOff = 4 * kABytes;
   static constexpr int kBarOff = kBOff + kKtStages * kBBytes;
-  // a_full, b_full[2], s_full[2], s_empty[2], a_empty
-  static constexpr int kMiscOff = kBarOff + 8 * 8;
+  // a_full[2], a_empty[2], b_full[3], b_empty[3], s_full[2][2] (token tile, accumulator), s_empty[2][2]
+  static constexpr int kMiscOff = kBarOff + 8 * (4 + 2 * kKtStages + 8);
   static constexpr int kTotal = kMiscOff + 16;
 };
 
@@ -104,17 +113,17 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
     return;
   }
   const uint32_t a_s = sbase + L::kAOff, b_s = sbase + L::kBOff, bars = sbase + L::kBarOff;
-  const uint32_t bar_a_full = bars, bar_b_full = bars + 8, bar_s_full = bars + 24, bar_s_empty = bars + 40, bar_a_empty = bars + 56;
+  const uint32_t bar_a_full = bars, bar_a_empty = bars + 16, bar_b_full = bars + 32, bar_b_empty = bar_b_full + 8 * kKtStages;
+  const uint32_t bar_s_full = bar_b_empty + 8 * kKtStages, bar_s_empty = bar_s_full + 32;
   volatile uint32_t* tmem_base_s = reinterpret_cast<volatile uint32_t*>(smem + L::kMiscOff);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(smem + L::kMiscOff + 4);
   const int ntiles = (p.num_centroids + kKtCent - 1) / kKtCent;
 
   if (threadIdx.x == 0) {
     *cta_abort = 0;
-    mbar_init(bar_a_full, 1);
-    for (int i = 0; i < kKtStages; ++i) mbar_init(bar_b_full + 8 * i, 1);
-    for (int a = 0; a < 2; ++a) { mbar_init(bar_s_full + 8 * a, 1); mbar_init(bar_s_empty + 8 * a, 128); }
-    mbar_init(bar_a_empty, 256);
+    for (int i = 0; i < 2; ++i) { mbar_init(bar_a_full + 8 * i, 1); mbar_init(bar_a_empty + 8 * i, 8 + 1); }   // epilogue warps, tensor core
+    for (int i = 0; i < 2 * kKtStages; ++i) mbar_init(bar_b_full + 8 * i, 1);
+    for (int i = 0; i < 4; ++i) { mbar_init(bar_s_full + 8 * i, 1); mbar_init(bar_s_empty + 8 * i, 4); }
     fence_barrier_init();
     fence_proxy_async();
   }
@@ -137,24 +146,23 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
       for (long long it = blockIdx.x; ok && it < items; it += gridDim.x, ++n) {
         const int g = static_cast<int>(it / per_group), t0 = static_cast<int>(it % per_group) * kKtTokens;
         for (int j = 0; ok && j < ntiles; ++j, ++step) {
-          const int st = step & 1;
-          // stage st was last read by the MMAs of step - 2, token tile 1: their completion is s_full[1], phase step - 2
-          if (step >= 2) ok = mbar_wait(bar_s_full + 8, (step - 2) & 1, cta_abort, 401);
+          const int st = step % kKtStages;
+          if (step >= kKtStages) ok = mbar_wait(bar_b_empty + 8 * st, (step / kKtStages - 1) & 1, cta_abort, 401);
           if (!ok) break;
           mbar_expect_tx(bar_b_full + 8 * st, L::kBBytes);
 #pragma unroll
           for (int h = 0; h < D / 64; ++h)
             tma_load_4d(b_s + st * L::kBBytes + h * (kKtCent * 128), &tm_cent, bar_b_full + 8 * st, h * 64, j * kKtCent, g, 0);
           if (j == 0) {
-            // the token tiles were last read by the MMAs of the previous step and by the epilogue (their norms)
-            if (n >= 1) ok = mbar_wait(bar_s_full + 8, (step - 1) & 1, cta_abort, 402) && mbar_wait(bar_a_empty, (n - 1) & 1, cta_abort, 403);
+            const uint32_t ab = n & 1;   // an item's token tiles arrive while the one before it is worked on
+            if (n >= 2) ok = mbar_wait(bar_a_empty + 8 * ab, ((n >> 1) - 1) & 1, cta_abort, 403);
             if (!ok) break;
-            mbar_expect_tx(bar_a_full, 2 * L::kABytes);
+            mbar_expect_tx(bar_a_full + 8 * ab, 2 * L::kABytes);
 #pragma unroll
             for (int a = 0; a < 2; ++a)
 #pragma unroll
               for (int h = 0; h < D / 64; ++h)
-                tma_load_4d(a_s + a * L::kABytes + h * (128 * 128), &tm_data, bar_a_full, h * 64, t0 + a * 128, g, 0);
+                tma_load_4d(a_s + (2 * ab + a) * L::kABytes + h * (128 * 128), &tm_data, bar_a_full + 8 * ab, h * 64, t0 + a * 128, g, 0);
           }
         }
       }
@@ -167,26 +175,29 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
       bool ok = true;
       uint32_t step = 0, n = 0;
       for (long long it = blockIdx.x; ok && it < items; it += gridDim.x, ++n) {
-        ok = mbar_wait_warp(bar_a_full, n & 1, cta_abort, 411);
+        const uint32_t ab = n & 1;
+        ok = mbar_wait_warp(bar_a_full + 8 * ab, (n >> 1) & 1, cta_abort, 411);
         for (int j = 0; ok && j < ntiles; ++j, ++step) {
-          const int st = step & 1;
-          ok = mbar_wait_warp(bar_b_full + 8 * st, (step >> 1) & 1, cta_abort, 412);
+          const int st = step % kKtStages, buf = step & 1;
+          ok = mbar_wait_warp(bar_b_full + 8 * st, (step / kKtStages) & 1, cta_abort, 412);
           if (!ok) break;
           const uint64_t b_desc = smem_desc_sw128(b_s + st * L::kBBytes, 16, 1024);
           for (int a = 0; ok && a < 2; ++a) {
-            if (step >= 1) ok = mbar_wait_warp(bar_s_empty + 8 * a, (step - 1) & 1, cta_abort, 413);
+            if (step >= 2) ok = mbar_wait_warp(bar_s_empty + 16 * a + 8 * buf, ((step >> 1) - 1) & 1, cta_abort, 413);
             if (!ok) break;
             tc_fence_after();
-            const uint64_t a_desc = smem_desc_sw128(a_s + a * L::kABytes, 16, 1024);
+            const uint64_t a_desc = smem_desc_sw128(a_s + (2 * ab + a) * L::kABytes, 16, 1024);
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
               const uint32_t off_a = (kk >> 2) * (128 * 128) + (kk & 3) * 32;
               const uint32_t off_b = (kk >> 2) * (kKtCent * 128) + (kk & 3) * 32;
-              mma_ss_elect(tmem + a * kKtCent, a_desc + (off_a >> 4), b_desc + (off_b >> 4), idesc, kk > 0);
+              mma_ss_elect(tmem + (2 * a + buf) * kKtCent, a_desc + (off_a >> 4), b_desc + (off_b >> 4), idesc, kk > 0);
             }
-            tc_commit_elect(bar_s_full + 8 * a);
+            tc_commit_elect(bar_s_full + 16 * a + 8 * buf);
           }
+          tc_commit_elect(bar_b_empty + 8 * st);
         }
+        tc_commit_elect(bar_a_empty + 8 * ab);
       }
     }
   } else {
@@ -195,17 +206,23 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
     const int quarter = warp & 3;               // TMEM lanes this warp may touch: 32 * (warp % 4) ..
     const int row = quarter * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    uint32_t keep = ~31u;                       // a score's low five bits make room for its column in the chunk
-    asm volatile("" : "+r"(keep));              // in a register: one three-input logic operation per score
+    uint64_t column[16];                        // 32nds, for two scores at a time
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      column[c] = f32x2_pack(2 * c / 32.0f, (2 * c + 1) / 32.0f);
+      asm volatile("" : "+l"(column[c]));       // in registers, not loaded for every use
+    }
+    const uint64_t whole = f32x2_pack(12582912.0f, 12582912.0f);
     bool ok = true;
     uint32_t step = 0, n = 0;
     for (long long it = blockIdx.x; it < items; it += gridDim.x, ++n) {
       const int g = static_cast<int>(it / per_group), tok = static_cast<int>(it % per_group) * kKtTokens + a * 128 + row;
       // |k|^2 of this thread's token, from the staged tile (16-byte chunk c of a row sits at c ^ (row & 7))
-      ok = mbar_wait_warp(bar_a_full, n & 1, cta_abort, 420);
+      const uint32_t ab = n & 1;
+      ok = mbar_wait_warp(bar_a_full + 8 * ab, (n >> 1) & 1, cta_abort, 420);
       if (!ok) break;
       float nrm2 = 0.f;
-      const uint8_t* arow = smem + L::kAOff + a * L::kABytes + row * 128;
+      const uint8_t* arow = smem + L::kAOff + (2 * ab + a) * L::kABytes + row * 128;
 #pragma unroll
       for (int ch = 0; ch < D / 8; ++ch) {
         const uint4 raw = *reinterpret_cast<const uint4*>(arow + (ch >> 3) * (128 * 128) + (((ch & 7) ^ (row & 7)) << 4));
@@ -214,23 +231,29 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
 #pragma unroll
         for (int i = 0; i < 8; ++i) nrm2 += f[i] * f[i];
       }
-      mbar_arrive(bar_a_empty);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_a_empty + 8 * ab);
+      const float scale = kKtScale / (sqrtf(nrm2) * sqrtf(p.max_cnorm2[g]));
+      const uint64_t scale2 = f32x2_pack(scale, scale);
       float best = -INFINITY, second = -INFINITY;
       int best_chunk = 0;
       for (int j = 0; ok && j < ntiles; ++j, ++step) {
-        ok = mbar_wait_warp(bar_s_full + 8 * a, step & 1, cta_abort, 421);
+        const int buf = step & 1;
+        ok = mbar_wait_warp(bar_s_full + 16 * a + 8 * buf, (step >> 1) & 1, cta_abort, 421);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t s_tmem = tmem + lane_addr + a * kKtCent;
+        const uint32_t s_tmem = tmem + lane_addr + (2 * a + buf) * kKtCent;
         // num_centroids is a multiple of 32: a 32-column chunk is whole or absent
         const int nch = min(kKtCent / 32, (p.num_centroids - j * kKtCent) / 32);
-        // The column rides in the score's low bits, so the running maximum carries it along: two scores that differ by
-        // less than that are re-scored anyway.  Two at a time: the larger against the best, the rest against the second.
+        // The column rides in the score's 32nds, so the running maximum carries it along.  Two at a time: the larger against
+        // the best, the rest against the second.
         auto scan = [&](const uint32_t (&r)[32], int chunk) {
           const float before = best;
 #pragma unroll
           for (int c = 0; c < 32; c += 2) {
-            const float v0 = __uint_as_float((r[c] & keep) | c), v1 = __uint_as_float((r[c + 1] & keep) | (c + 1));
+            float v0, v1;
+            const uint64_t u = f32x2_fma(f32x2_pack(__uint_as_float(r[c]), __uint_as_float(r[c + 1])), scale2, whole);
+            f32x2_unpack(f32x2_add(f32x2_sub(u, whole), column[c / 2]), v0, v1);
             const float hi = fmaxf(v0, v1), lo = fminf(v0, v1);
             second = max3(second, lo, fminf(best, hi));
             best = fmaxf(best, hi);
@@ -239,29 +262,35 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
         };
         // two register buffers: the load of the next chunk is in flight while this one is scanned
         uint32_t r0[32], r1[32];
+        const int chunk0 = j * (kKtCent / 32);
         tmem_ld32(s_tmem, r0);
-#pragma unroll 1
-        for (int ch = 0; ch < nch; ch += 2) {
-          tmem_wait_ld();
-          if (ch + 1 < nch) tmem_ld32(s_tmem + (ch + 1) * 32, r1);
-          scan(r0, j * (kKtCent / 32) + ch);
-          if (ch + 1 < nch) {
+        if (nch == kKtCent / 32) {
+#pragma unroll
+          for (int ch = 0; ch < kKtCent / 32; ch += 2) {
             tmem_wait_ld();
-            if (ch + 2 < nch) tmem_ld32(s_tmem + (ch + 2) * 32, r0);
-            scan(r1, j * (kKtCent / 32) + ch + 1);
+            tmem_ld32(s_tmem + (ch + 1) * 32, r1);
+            scan(r0, chunk0 + ch);
+            tmem_wait_ld();
+            if (ch + 2 < kKtCent / 32) tmem_ld32(s_tmem + (ch + 2) * 32, r0);
+            scan(r1, chunk0 + ch + 1);
+          }
+        } else {
+#pragma unroll 1
+          for (int ch = 0; ch < nch; ++ch) {
+            tmem_wait_ld();
+            scan(r0, chunk0 + ch);
+            if (ch + 1 < nch) tmem_ld32(s_tmem + (ch + 1) * 32, r0);
           }
         }
         tc_fence_before();
-        mbar_arrive(bar_s_empty + 8 * a);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_s_empty + 16 * a + 8 * buf);
       }
       if (!ok) break;
       if (tok < p.num_tokens) {
         const long long at = static_cast<long long>(g) * p.num_tokens + tok;
-        const int best_idx = best_chunk * 32 + static_cast<int>(__float_as_uint(best) & 31u);
-        // the accumulation's error, and what the columns in the low bits can make of equal scores (31 units in the last
-        // place of each)
-        const float tol = kKtTol * sqrtf(nrm2) * sqrtf(p.max_cnorm2[g]) + 7.7e-6f * fabsf(best);
-        const bool sure = (best - second) > tol && fminf(nrm2, p.max_cnorm2[g]) >= kKtMinNorm2;
+        const int best_idx = best_chunk * 32 + (static_cast<int>(best * 32.0f) & 31);
+        const bool sure = (best - second) > kKtGap && fminf(nrm2, p.max_cnorm2[g]) >= kKtMinNorm2;
         p.idx[at] = sure ? best_idx : (-1 - best_idx);
         if (!sure) {
           const int slot = atomicAdd(p.flagged_count, 1);

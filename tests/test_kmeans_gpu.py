@@ -162,6 +162,20 @@ def test_assignment_over_many_items(dtype, g, t, k, d):
     assert torch.equal(counts.long(), torch.stack([torch.bincount(r.long(), minlength=k) for r in idx]))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("g,t,k,d", [(1, 300, 32, 128), (2, 700, 160, 64), (1, 513, 416, 128)])
+def test_assignment_among_negative_and_close_scores(dtype, g, t, k, d):
+    """Every score is negative and most lie within a few parts in a thousand of each other, so that the largest one is
+    a small negative number of the scan's units; exact arg-max, lowest index on ties."""
+    from longcontext_sqattn_paddle_b200.cache_hub import kmeans as km
+    gen = torch.Generator().manual_seed(31 * k + d)
+    data = (torch.rand(g, t, d, generator=gen) + 0.5).to(dtype)
+    cent = (-1.0 - 2.0 ** -6 * torch.rand(g, k, d, generator=gen)).to(dtype)
+    cent[:, k // 2:] = cent[:, : k - k // 2].roll(1, 2)
+    _, idx, _ = km.k_means_train(data.cuda(), cent.cuda().clone(), False)
+    assert torch.equal(idx.cpu(), ko.assign(data, cent).to(idx.dtype))
+
+
 @pytest.mark.parametrize("key_exp,cent_exp", [(0, 0), (-90, 0), (0, -90), (-80, -70), (100, 30)])
 @pytest.mark.parametrize("d", [64, 128])
 def test_assignment_where_fp32_has_no_squares_of_the_norms(d, key_exp, cent_exp):
