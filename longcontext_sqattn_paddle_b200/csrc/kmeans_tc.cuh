@@ -313,16 +313,20 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
   }
 }
 
-// Exact re-scoring of the listed tokens, one CTA per token at a time (the CTAs loop over the list):
-//   1. fp32 scores of ALL centroids of the group into shared memory, a half warp (D = 128) per centroid row with
-//      16-byte loads, so a token costs one coalesced sweep over its group's centroids;
-//   2. the candidates: centroids whose fp32 score lies within the error band of the largest one (the same bound
-//      as in the assignment kernel, which also covers this pass's own rounding); a score that is not a number counts;
+// Exact re-scoring of the listed tokens, up to kRecheckTokens consecutive ones of the list per CTA and sweep (the CTAs loop
+// over the list; neighbours in it mostly belong to one group, and a sweep serves those of one group):
+//   1. fp32 scores of ALL centroids of the group into shared memory: mma.sync m16n8k16 with 16 centroid rows as A, straight
+//      from global memory (16 bytes of a row per lane; the order of the channels inside a product does not matter), and the
+//      tokens as the columns of B.  A token's own sweep with fp32 FMAs took 15 instructions per row for unpacking and shuffles
+//      and one read of all centroids per token: 74 us for the 1600 or so tokens of an iteration (8 x 65536 keys, 1024 centroids), 33 us like this: latency of a sweep and of the fp64 chain;
+//   2. a warp per token: the candidates, i.e. centroids whose fp32 score lies within the error band of the largest one (the
+//      same bound as in the assignment kernel, which also covers this pass's own rounding); a score that is not a number counts;
 //   3. the candidates' exact scores in fp64 (exact products, index-order sum), the largest wins, the lowest index
 //      on ties.  More than kMaxCand candidates (degenerate data, e.g. an all-zero key) take the fp64 path for every
 //      centroid.
 // When the list overflowed, every token whose idx is still negative is re-scored instead (a sweep over all
 // tokens, the list is ignored).
+constexpr int kRecheckTokens = 8;
 constexpr int kMaxCand = 64;
 
 template <int D, bool BF16>
@@ -339,107 +343,117 @@ __device__ __forceinline__ double exact_score(const double* kd, const uint8_t* r
   return s;
 }
 
+// per_sweep <= kRecheckTokens: as many tokens as the scores' shared memory holds
 template <int D, bool BF16>
 __global__ void __launch_bounds__(256)
 kmeans_recheck_list_kernel(const uint8_t* data, const uint8_t* cent, int* idx, const int* flagged, const int* flagged_count,
-                           int flagged_cap, const float* max_cnorm2, int groups, int num_tokens, int num_centroids) {
-  extern __shared__ float score_s[];      // [num_centroids]
-  __shared__ double kd[D];
-  __shared__ float red_s[8];
-  __shared__ double best_s[8];
-  __shared__ int idx_s[8];
-  __shared__ int cand_s[kMaxCand];
-  __shared__ int ncand_s;
-  constexpr int kLanes = D / 8;           // lanes per centroid row
-  constexpr int kRows = 32 / kLanes;      // rows a warp takes at a time
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / kLanes, ch = lane % kLanes;
+                           int flagged_cap, const float* max_cnorm2, int groups, int num_tokens, int num_centroids, int per_sweep) {
+  extern __shared__ float score_s[];      // [per_sweep][num_centroids]
+  __shared__ double kd_s[kRecheckTokens][D];
+  __shared__ int cand_s[kRecheckTokens][kMaxCand];
+  __shared__ int token_s[kRecheckTokens];  // g * num_tokens + t, -1: none
+  static_assert(kRecheckTokens == 8, "a warp per token, a column of the matrix product per token");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int count = *flagged_count;
   const bool sweep = count > flagged_cap;
   const long long total = sweep ? static_cast<long long>(groups) * num_tokens : count;
-  for (long long e = blockIdx.x; e < total; e += gridDim.x) {
-    const long long at = sweep ? e : flagged[e];
-    if (sweep && idx[at] >= 0) continue;
-    const int g = static_cast<int>(at / num_tokens);
-    const uint8_t* krow = data + at * D * 2;
-    const uint8_t* cg = cent + static_cast<long long>(g) * num_centroids * D * 2;
+  for (long long e0 = static_cast<long long>(blockIdx.x) * per_sweep; e0 < total; e0 += static_cast<long long>(gridDim.x) * per_sweep) {
     __syncthreads();
-    float kf[8];
-    unpack8<BF16>(*reinterpret_cast<const uint4*>(krow + ch * 16), kf);
-    if (threadIdx.x < kLanes) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) kd[ch * 8 + i] = static_cast<double>(kf[i]);
-    }
-    if (threadIdx.x == 0) ncand_s = 0;
-    float nrm2 = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) nrm2 += kf[i] * kf[i];
-    for (int o = 1; o < kLanes; o <<= 1) nrm2 += __shfl_xor_sync(0xffffffffu, nrm2, o);
-    // 1. fp32 scores, four rows per half warp in flight
-    float mx = -INFINITY;
-    for (int c0 = warp * kRows + sub; c0 < num_centroids; c0 += 8 * kRows * 4) {
-      uint4 v[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int c = c0 + u * 8 * kRows;
-        v[u] = c < num_centroids ? *reinterpret_cast<const uint4*>(cg + (static_cast<long long>(c) * D + ch * 8) * 2)
-                                 : make_uint4(0, 0, 0, 0);
+    if (threadIdx.x < kRecheckTokens) {
+      const long long e = e0 + threadIdx.x;
+      int at = -1;
+      if (threadIdx.x < per_sweep && e < total) {
+        at = sweep ? static_cast<int>(e) : flagged[e];
+        if (sweep && idx[at] >= 0) at = -1;
       }
+      token_s[threadIdx.x] = at;
+    }
+    __syncthreads();
+    unsigned left = 0;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int c = c0 + u * 8 * kRows;
-        float f[8], sc = 0.f;
-        unpack8<BF16>(v[u], f);
+    for (int j = 0; j < kRecheckTokens; ++j) left |= token_s[j] >= 0 ? 1u << j : 0u;
+    while (left) {
+      // the tokens of the first one's group
+      const int g = token_s[__ffs(left) - 1] / num_tokens;
+      unsigned mine = 0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) sc += kf[i] * f[i];
-        for (int o = 1; o < kLanes; o <<= 1) sc += __shfl_xor_sync(0xffffffffu, sc, o);
-        if (c < num_centroids) {
-          if (ch == 0) score_s[c] = sc;
-          mx = fmaxf(mx, sc);
+      for (int j = 0; j < kRecheckTokens; ++j) mine |= (left >> j & 1u) && token_s[j] / num_tokens == g ? 1u << j : 0u;
+      left &= ~mine;
+      const uint8_t* cg = cent + static_cast<long long>(g) * num_centroids * D * 2;
+      // 1. lane (r, c) = (lane / 4, lane % 4) reads channels 8 (4 q + c) .. + 7: of token r for B, of rows r and r + 8 for A
+      const int r = lane >> 2, c = lane & 3;
+      uint4 b[D / 32];
+#pragma unroll
+      for (int q = 0; q < D / 32; ++q)
+        b[q] = mine >> r & 1u ? *reinterpret_cast<const uint4*>(data + (static_cast<long long>(token_s[r]) * D + 8 * (4 * q + c)) * 2)
+                              : make_uint4(0, 0, 0, 0);
+      for (int row0 = warp * 16; row0 < num_centroids; row0 += 8 * 16) {
+        uint4 a0[D / 32], a1[D / 32];
+        const uint8_t* row = cg + (static_cast<long long>(row0 + r) * D + 8 * c) * 2;
+#pragma unroll
+        for (int q = 0; q < D / 32; ++q) {
+          a0[q] = *reinterpret_cast<const uint4*>(row + q * 64);
+          a1[q] = *reinterpret_cast<const uint4*>(row + q * 64 + 8 * D * 2);
         }
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) red_s[warp] = mx;
-    __syncthreads();
-    mx = red_s[0];
-    for (int w = 1; w < 8; ++w) mx = fmaxf(mx, red_s[w]);
-    // 2. candidates inside the error band; without a band (norms beyond fp32 squares either way) none is left out
-    const float cnorm2 = max_cnorm2[g];
-    const float tol = fminf(nrm2, cnorm2) >= kKtMinNorm2 ? kKtTol * sqrtf(nrm2) * sqrtf(cnorm2) : INFINITY;
-    for (int c = threadIdx.x; c < num_centroids; c += 256) {
-      if (!(score_s[c] < mx - tol)) {
-        const int slot = atomicAdd(&ncand_s, 1);
-        if (slot < kMaxCand) cand_s[slot] = c;
-      }
-    }
-    __syncthreads();
-    const int ncand = ncand_s;
-    // 3. exact scores
-    double best = -1.0 / 0.0;
-    int bi = 0x7fffffff;
-    if (ncand <= kMaxCand) {
-      if (threadIdx.x < ncand) {
-        bi = cand_s[threadIdx.x];
-        best = exact_score<D, BF16>(kd, cg + static_cast<long long>(bi) * D * 2);
-      }
-    } else {
-      for (int c = threadIdx.x; c < num_centroids; c += 256) {
-        const double sc = exact_score<D, BF16>(kd, cg + static_cast<long long>(c) * D * 2);
-        if (sc > best) { best = sc; bi = c; }   // ascending c: the lowest index is kept on ties
-      }
-    }
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-    }
-    if (lane == 0) { best_s[warp] = best; idx_s[warp] = bi; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int w = 1; w < 8; ++w)
-        if (best_s[w] > best || (best_s[w] == best && idx_s[w] < bi)) { best = best_s[w]; bi = idx_s[w]; }
-      idx[at] = bi < num_centroids ? bi : 0;   // no candidate at all: a NaN key
+        for (int q = 0; q < D / 32; ++q) {
+          const uint32_t lo[4] = {a0[q].x, a1[q].x, a0[q].y, a1[q].y}, hi[4] = {a0[q].z, a1[q].z, a0[q].w, a1[q].w};
+          mma_16816<BF16>(s, lo, b[q].x, b[q].y);
+          mma_16816<BF16>(s, hi, b[q].z, b[q].w);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)   // rows r, r, r + 8, r + 8 of tokens 2 c, 2 c + 1
+          if (mine >> (2 * c + (i & 1)) & 1u) score_s[(2 * c + (i & 1)) * num_centroids + row0 + r + 8 * (i >> 1)] = s[i];
+      }
+      // the token as fp64, and its norm
+      float nrm2 = 0.f;
+      if (mine >> warp & 1u) {
+        const uint8_t* krow = data + static_cast<long long>(token_s[warp]) * D * 2;
+        for (int ch = lane; ch < D; ch += 32) {
+          const float f = to_f32<BF16>(reinterpret_cast<const uint16_t*>(krow)[ch]);
+          kd_s[warp][ch] = static_cast<double>(f);
+          nrm2 += f * f;
+        }
+        for (int o = 16; o > 0; o >>= 1) nrm2 += __shfl_xor_sync(0xffffffffu, nrm2, o);
+      }
+      __syncthreads();
+      if (mine >> warp & 1u) {
+        const float* score = score_s + warp * num_centroids;
+        const double* kd = kd_s[warp];
+        // 2. candidates inside the error band; without a band (norms beyond fp32 squares either way) none is left out
+        float mx = -INFINITY;
+        for (int k = lane; k < num_centroids; k += 32) mx = fmaxf(mx, score[k]);
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float cnorm2 = max_cnorm2[g];
+        const float tol = fminf(nrm2, cnorm2) >= kKtMinNorm2 ? kKtTol * sqrtf(nrm2) * sqrtf(cnorm2) : INFINITY;
+        int ncand = 0;
+        for (int k = lane; k < num_centroids; k += 32) {   // num_centroids is a multiple of 32
+          const bool near = !(score[k] < mx - tol);
+          const unsigned votes = __ballot_sync(0xffffffffu, near);
+          const int slot = ncand + __popc(votes & ((1u << lane) - 1u));
+          if (near && slot < kMaxCand) cand_s[warp][slot] = k;
+          ncand += __popc(votes);
+        }
+        __syncwarp();
+        // 3. exact scores; a lane's centroids ascend, so the lowest index is kept on ties
+        double best = -1.0 / 0.0;
+        int bi = 0x7fffffff;
+        const bool listed = ncand <= kMaxCand;
+        for (int k = lane; k < (listed ? ncand : num_centroids); k += 32) {
+          const int cand = listed ? cand_s[warp][k] : k;
+          const double sc = exact_score<D, BF16>(kd, cg + static_cast<long long>(cand) * D * 2);
+          if (sc > best || (sc == best && cand < bi)) { best = sc; bi = cand; }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+          const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+          if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+        }
+        if (lane == 0) idx[token_s[warp]] = bi < num_centroids ? bi : 0;   // no candidate at all: a NaN key
+      }
+      __syncthreads();
     }
   }
 }

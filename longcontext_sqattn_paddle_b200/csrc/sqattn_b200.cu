@@ -809,7 +809,9 @@ int sqattn_kmeans_assign(const void* data, const void* centroids, int32_t dtype,
                             : km_launch_assign<64>(data, centroids, dtype, groups, num_tokens, num_centroids, idx, w, stream)))
     return rc;
   {
-    const int smem = num_centroids * static_cast<int>(sizeof(float));   // the fp32 scores of one group
+    int per_sweep = kRecheckTokens;   // the fp32 scores of a sweep's tokens: 192 KB at most
+    while (static_cast<long long>(per_sweep) * num_centroids > 49152) per_sweep /= 2;
+    const int smem = per_sweep * num_centroids * static_cast<int>(sizeof(float));
     if (head_dim == 128) {
       if (bf16) SQ_CUDA(cudaFuncSetAttribute(kmeans_recheck_list_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       else SQ_CUDA(cudaFuncSetAttribute(kmeans_recheck_list_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -818,7 +820,7 @@ int sqattn_kmeans_assign(const void* data, const void* centroids, int32_t dtype,
       else SQ_CUDA(cudaFuncSetAttribute(kmeans_recheck_list_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     }
     SQ_KM_DISPATCH(kmeans_recheck_list_kernel, <<<148 * 4, 256, smem, stream>>>(d8, c8, idx, w.flagged, w.flagged_count, w.flagged_cap,
-                                                                             w.max_cnorm2, groups, num_tokens, num_centroids));
+                                                                             w.max_cnorm2, groups, num_tokens, num_centroids, per_sweep));
   }
   SQ_CUDA(cudaGetLastError());
   if (sums) {
