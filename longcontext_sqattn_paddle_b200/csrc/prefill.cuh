@@ -411,6 +411,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
           for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(f[e]));
         }
         amax = fmaxf(amax, 1e-5f);
+        const float scale = __fdiv_rn(amax, 127.0f), inv = __fdiv_rn(1.0f, scale);
         const int qtype = p.q_fake_quant - 1;
 #pragma unroll
         for (int ch = 0; ch < D / 8; ++ch) {
@@ -418,8 +419,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
           uint4 outv;
           if (p.qk_bf16) unpack8<true>(raw[ch], f); else unpack8<false>(raw[ch], f);
           if (qtype == SQATTN_QTYPE_INT) {
-            outv = p.qk_bf16 ? fake_quant_int_row8<true, true>(f, amax, 127.0f, p.q_half_even, p.q_scale)
-                             : fake_quant_int_row8<false, true>(f, amax, 127.0f, p.q_half_even, p.q_scale);
+            outv = p.qk_bf16 ? fake_quant_int_row8<true, true>(raw[ch], scale, inv, 127.0f, p.q_half_even, p.q_scale)
+                             : fake_quant_int_row8<false, true>(raw[ch], scale, inv, 127.0f, p.q_half_even, p.q_scale);
           } else {
             float g[8];
 #pragma unroll

@@ -51,29 +51,28 @@ struct OutStrides {  // element strides of an output [B,H,N,D] (contiguous HND o
 // out (contiguous [B,H,N,D]) = f(in): kOp 0: x * scale rounded to the input dtype (q pre-scaling,
 // attn_triton_mix_relative.py:383-385); kOp 1: bf16 -> f16 (the kernel-side v.to(fp16), attn_triton.py:84).
 template <bool BF16, int kOp>
-__global__ void strided_map_kernel(View4 in, uint8_t* out, float scale) {
-  const int d8 = in.d / 8;
-  const long long total = static_cast<long long>(in.b) * in.h * in.n * d8;
-  for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
-       idx += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int c = static_cast<int>(idx % d8);
-    long long r = idx / d8;
-    const int n = static_cast<int>(r % in.n);
-    r /= in.n;
-    const int h = static_cast<int>(r % in.h);
-    const int b = static_cast<int>(r / in.h);
-    const uint4 v = *reinterpret_cast<const uint4*>(in.ptr + 2 * (b * in.sb + h * in.sh + n * in.sn + c * 8));
-    float f[8];
-    unpack8<BF16>(v, f);
-    uint4 o;
-    if (kOp == 0) {
+__global__ void __launch_bounds__(256) strided_map_kernel(View4 in, uint8_t* out, float scale) {
+  // a (batch, head) per blockIdx.y: no division but the shift by d / 8 in a thread's loop
+  const int shift = in.d == 128 ? 4 : 3;
+  const long long per = static_cast<long long>(in.n) << shift;
+  for (int bh = blockIdx.y; bh < in.b * in.h; bh += gridDim.y) {
+    const uint8_t* src = in.ptr + 2 * (bh / in.h * in.sb + bh % in.h * in.sh);
+    uint8_t* dst = out + bh * per * 16;
+    for (long long idx = blockIdx.x * 256ll + threadIdx.x; idx < per; idx += gridDim.x * 256ll) {
+      const int c = static_cast<int>(idx) & ((1 << shift) - 1);
+      const uint4 v = *reinterpret_cast<const uint4*>(src + 2 * ((idx >> shift) * in.sn + c * 8));
+      float f[8];
+      unpack8<BF16>(v, f);
+      uint4 o;
+      if (kOp == 0) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] *= scale;
-      o = pack8<BF16>(f);
-    } else {
-      o = pack8<false>(f);
+        for (int i = 0; i < 8; ++i) f[i] *= scale;
+        o = pack8<BF16>(f);
+      } else {
+        o = pack8<false>(f);
+      }
+      *reinterpret_cast<uint4*>(dst + idx * 16) = o;
     }
-    *reinterpret_cast<uint4*>(out + idx * 16) = o;
   }
 }
 
@@ -147,16 +146,18 @@ __device__ __forceinline__ float float_quantize_dev(float x, int e_bits, int m_b
   return fminf(fmaxf(xq, -max_val), max_val);
 }
 
+// quant -> dequant of one value on the integer grid of `scale`, with the reference's divisions
+__device__ __forceinline__ float int_grid_value(float x, float scale, float qmax, int half_even) {
+  float q = round_mode(__fdiv_rn(x, scale), half_even);
+  q = fminf(fmaxf(q, -qmax - 1.0f), qmax);
+  return q * scale;
+}
+
 // quant -> dequant of one value given the row's absmax (clipped at 1e-5).
 //   qtype 0: integer grid with `qmax` (127 / 7), clamp to [-qmax-1, qmax]  (fake_quant.py:114-125)
 //   qtype 1/2: emulated e4m3 / e5m2                                         (fake_quant.py:231-248)
 __device__ __forceinline__ float fake_quant_value(float x, float absmax, int qtype, float qmax, int half_even) {
-  if (qtype == SQATTN_QTYPE_INT) {
-    const float scale = __fdiv_rn(absmax, qmax);
-    float q = round_mode(__fdiv_rn(x, scale), half_even);
-    q = fminf(fmaxf(q, -qmax - 1.0f), qmax);
-    return q * scale;
-  }
+  if (qtype == SQATTN_QTYPE_INT) return int_grid_value(x, __fdiv_rn(absmax, qmax), qmax, half_even);
   const float fmax = (qtype == SQATTN_QTYPE_E4M3) ? 448.0f : 57344.0f;
   const float scale = __fdiv_rn(absmax, fmax);
   float s = fminf(fmaxf(__fdiv_rn(x, scale), -fmax), fmax);
@@ -164,61 +165,78 @@ __device__ __forceinline__ float fake_quant_value(float x, float absmax, int qty
   return s * scale;
 }
 
-// rintf of two values below 2^22 in magnitude: adding and taking off 1.5 * 2^23 leaves the nearest integer (ties to even),
-// the sign goes back on for the negative zeros.  The conversion unit's own rounding runs at an eighth of this rate.
+// The nearest integers of two values below 2^22 in magnitude: adding and taking off 1.5 * 2^23 leaves them (ties to even; a
+// negative zero comes out positive).  The conversion unit's own rounding runs at an eighth of this rate.
 __device__ __forceinline__ uint64_t rint2_small(uint64_t x2) {
   const uint64_t m = f32x2_pack(12582912.0f, 12582912.0f);
-  float a, b, r0, r1;
-  f32x2_unpack(x2, a, b);
-  f32x2_unpack(f32x2_sub(f32x2_add(x2, m), m), r0, r1);
-  return f32x2_pack(copysignf(r0, a), copysignf(r1, b));
+  return f32x2_sub(f32x2_add(x2, m), m);
+}
+template <bool BF16>
+__device__ __forceinline__ void unpack2(uint32_t w, float& lo, float& hi) {
+  lo = to_f32<BF16>(static_cast<uint16_t>(w & 0xffffu));
+  hi = BF16 ? __uint_as_float(w & 0xffff0000u) : to_f32<BF16>(static_cast<uint16_t>(w >> 16));
+}
+template <bool BF16>
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) { return BF16 ? pack_bf16x2(lo, hi) : pack_f16x2(lo, hi); }
+// largest magnitude of 8 values, in their own type (a NaN counts as nothing beside a number)
+template <bool BF16>
+__device__ __forceinline__ float absmax8(const uint4& x) {
+  auto larger = [](uint32_t a, uint32_t b) {
+    uint32_t r;
+    if (BF16) asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    else asm("max.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+  };
+  constexpr uint32_t kAbs = 0x7fff7fffu;
+  float lo, hi;
+  unpack2<BF16>(larger(larger(x.x & kAbs, x.y & kAbs), larger(x.z & kAbs, x.w & kAbs)), lo, hi);
+  return fmaxf(lo, hi);
 }
 
-// The integer grid for the 8 values a thread holds of one row, on packed fp32 pairs, returning the 8 results
+// The integer grid for 8 values of one row, on packed fp32 pairs, returning the 8 results
 // rounded to the 16-bit type (and, for queries, multiplied by q_scale and rounded again) as four packed words.
-// q = x * (1/scale) is within 2e-5 of the exact quotient x / scale (|q| <= qmax * (1 + 2^-22), so the clamp of the
+// q = x * inv, inv = 1/scale, is within 2e-5 of the exact quotient x / scale (|q| <= qmax * (1 + 2^-22), so the clamp of the
 // reference never acts), hence unless q lies within 1e-4 of a half-integer its nearest integer IS round(x / scale) in
 // either rounding mode; a group with such a value (rare) is redone with exact divisions.  The bits are those of
-// fake_quant_value(..., INT, ...).
+// fake_quant_value(..., INT, ...).  A result has the sign of its input, zeros too: the sign bits are put back two at a time.
 template <bool BF16, bool kScale>
-__device__ __forceinline__ uint4 fake_quant_int_row8(const float (&x)[8], float absmax, float qmax, int half_even, float q_scale) {
-  const float scale = __fdiv_rn(absmax, qmax), inv = __fdiv_rn(1.0f, scale);
+__device__ __forceinline__ uint4 fake_quant_int_row8(const uint4& x, float scale, float inv, float qmax, int half_even, float q_scale) {
   const uint64_t inv2 = f32x2_pack(inv, inv), sc2 = f32x2_pack(scale, scale), qs2 = f32x2_pack(q_scale, q_scale);
+  const uint32_t w[4] = {x.x, x.y, x.z, x.w};
   float g[8];
   float worst = 0.f;
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
-    const uint64_t q2 = f32x2_mul(f32x2_pack(x[2 * p], x[2 * p + 1]), inv2);
-    float d0, d1;
+    float a, b, d0, d1;
+    unpack2<BF16>(w[p], a, b);
+    const uint64_t q2 = f32x2_mul(f32x2_pack(a, b), inv2);
     const uint64_t r2 = rint2_small(q2);
     f32x2_unpack(f32x2_sub(q2, r2), d0, d1);
-    worst = fmaxf(worst, fmaxf(fabsf(d0), fabsf(d1)));
+    worst = max3(worst, fabsf(d0), fabsf(d1));
     f32x2_unpack(f32x2_mul(r2, sc2), g[2 * p], g[2 * p + 1]);
   }
   if (worst > 0.4999f) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) g[i] = fake_quant_value(x[i], absmax, SQATTN_QTYPE_INT, qmax, half_even);
+    for (int p = 0; p < 4; ++p) {
+      float a, b;
+      unpack2<BF16>(w[p], a, b);
+      g[2 * p] = int_grid_value(a, scale, qmax, half_even);
+      g[2 * p + 1] = int_grid_value(b, scale, qmax, half_even);
+    }
   }
-  uint32_t w[4];
+  uint32_t out[4];
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
-    uint32_t v = BF16 ? pack_bf16x2(g[2 * p], g[2 * p + 1]) : pack_f16x2(g[2 * p], g[2 * p + 1]);
+    uint32_t v = pack2<BF16>(g[2 * p], g[2 * p + 1]);
     if (kScale) {
       float a, b;
-      if (BF16) {
-        a = __uint_as_float(v << 16);
-        b = __uint_as_float(v & 0xffff0000u);
-      } else {
-        const __half2 h2 = *reinterpret_cast<const __half2*>(&v);
-        a = __low2float(h2);
-        b = __high2float(h2);
-      }
+      unpack2<BF16>(v, a, b);
       f32x2_unpack(f32x2_mul(f32x2_pack(a, b), qs2), a, b);
-      v = BF16 ? pack_bf16x2(a, b) : pack_f16x2(a, b);
+      v = pack2<BF16>(a, b);
     }
-    w[p] = v;
+    out[p] = v | (w[p] & 0x80008000u);
   }
-  return make_uint4(w[0], w[1], w[2], w[3]);
+  return make_uint4(out[0], out[1], out[2], out[3]);
 }
 
 // "per_channel" fake-quant of V for the 4 channels c of token n: one range per (token, channel), taken over batch and
@@ -325,7 +343,6 @@ __device__ __forceinline__ void quant_rows_body(const QuantRows& r, const float*
   const int d8 = x.d / 8;
   const int rows_per_block = 256 / d8;
   const int c = threadIdx.x % d8;
-  const unsigned grp_mask = (d8 == 16) ? (0xffffu << ((threadIdx.x & 16) ? 16 : 0)) : (0xffu << ((threadIdx.x & 31) / 8 * 8));
   const int b = bh / x.h, h = bh % x.h;
   const uint8_t* in_base = x.ptr + 2 * (b * x.sb + h * x.sh + c * 8);
   const long long out_base = (b * r.os.sb + h * r.os.sh + c * 8) * 2;
@@ -341,45 +358,63 @@ __device__ __forceinline__ void quant_rows_body(const QuantRows& r, const float*
     const int n = n0 + u * rows_per_block;
     raw[u] = n < x.n ? *reinterpret_cast<const uint4*>(in_base + 2 * (static_cast<long long>(n) * x.sn)) : make_uint4(0u, 0u, 0u, 0u);
   }
+  float amax[kUnroll];
 #pragma unroll
   for (int u = 0; u < kUnroll; ++u) {
-    const int n = n0 + u * rows_per_block;
-    float f[8];
-    unpack8<BF16>(raw[u], f);
     if (kIsK) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] = to_f32<BF16>(from_f32<BF16>(f[i] - mvals[i]));
+      float f[8];
+      unpack8<BF16>(raw[u], f);
+      raw[u] = make_uint4(pack2<BF16>(f[0] - mvals[0], f[1] - mvals[1]), pack2<BF16>(f[2] - mvals[2], f[3] - mvals[3]),
+                          pack2<BF16>(f[4] - mvals[4], f[5] - mvals[5]), pack2<BF16>(f[6] - mvals[6], f[7] - mvals[7]));
     }
-    float amax = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
-    for (int o = d8 / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(grp_mask, amax, o));
-    amax = fmaxf(amax, 1e-5f);
-    if (n < x.n) {
-      const long long ooff = out_base + static_cast<long long>(n) * r.os.sn * 2;
-      if (kInt) {
-        *reinterpret_cast<uint4*>(r.out8 + ooff) = fake_quant_int_row8<BF16, !kIsK>(f, amax, 127.0f, half_even, q_scale);
-      } else {
-        float g[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          g[i] = to_f32<BF16>(from_f32<BF16>(fake_quant_value(f[i], amax, qtype, 127.0f, half_even)));
-          if (!kIsK) g[i] *= q_scale;
-        }
-        *reinterpret_cast<uint4*>(r.out8 + ooff) = pack8<BF16>(g);
-      }
-      if (r.out4) *reinterpret_cast<uint4*>(r.out4 + ooff) = fake_quant_int_row8<BF16, !kIsK>(f, amax, 7.0f, half_even, q_scale);
-    }
+    amax[u] = absmax8<BF16>(raw[u]);
   }
+  // The largest of each row over its lanes, transposed: lane c ends up with row c & 3 and is the one that divides for it.
+  static_assert(kUnroll == 4, "two exchange steps");
+  {
+    const bool b0 = c & 1, b1 = c & 2;
+    const float k0 = fmaxf(b0 ? amax[1] : amax[0], __shfl_xor_sync(0xffffffffu, b0 ? amax[0] : amax[1], 1));
+    const float k1 = fmaxf(b0 ? amax[3] : amax[2], __shfl_xor_sync(0xffffffffu, b0 ? amax[2] : amax[3], 1));
+    amax[0] = fmaxf(b1 ? k1 : k0, __shfl_xor_sync(0xffffffffu, b1 ? k0 : k1, 2));
+    for (int o = 4; o < d8; o <<= 1) amax[0] = fmaxf(amax[0], __shfl_xor_sync(0xffffffffu, amax[0], o));
+  }
+  const float mine = fmaxf(amax[0], 1e-5f);
+  const int src = threadIdx.x & 28;   // the lane of the group of four that has row u is src + u
+  auto rows = [&](uint8_t* out, float qmax, bool grid) {
+    const float scale = grid ? __fdiv_rn(mine, qmax) : mine, inv = grid ? __fdiv_rn(1.0f, scale) : 0.f;
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const int n = n0 + u * rows_per_block;
+      const float s = __shfl_sync(0xffffffffu, scale, src + u), i = __shfl_sync(0xffffffffu, inv, src + u);
+      uint4 v;
+      if (grid) {
+        v = fake_quant_int_row8<BF16, !kIsK>(raw[u], s, i, qmax, half_even, q_scale);
+      } else {
+        float f[8];
+        unpack8<BF16>(raw[u], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          f[e] = to_f32<BF16>(from_f32<BF16>(fake_quant_value(f[e], s, qtype, qmax, half_even)));
+          if (!kIsK) f[e] *= q_scale;
+        }
+        v = pack8<BF16>(f);
+      }
+      if (n < x.n) *reinterpret_cast<uint4*>(out + out_base + static_cast<long long>(n) * r.os.sn * 2) = v;
+    }
+  };
+  rows(r.out8, 127.0f, kInt);
+  if (r.out4) rows(r.out4, 7.0f, true);
 }
 
 // Preparation, second launch: the rows of Q (first: they do not wait for the first launch) and of K.  K blocks add up the
 // column sums of the first launch themselves, in chunk order, unless the caller gave the mean.
 // One launch for both, and V beside the sums, instead of five in a row, each of the small ones waiting for its own latency.
-// Rows are bound by instruction issue (about 12 per element), so blocks per SM count: five (48 registers, a few spilled).
-// In a graph, before and after, 28/4 heads: 1000 tokens 23.8 and 14.6 us, 8192 73 and 54, 131072 898 and 775 (2.4 TB/s).
+// A row's divisions are done by one of its lanes and passed on, its largest magnitude is found in the 16-bit type, and signs go
+// back on two at a time: every lane of a row divided for itself before (131072 tokens, queries alone: 540 -> 475 us, 4.0 TB/s).
+// Four blocks per SM (64 registers); five (48 registers, 300 bytes spilled) were 1 % slower, three 9 %.
+// In a graph, five launches, two, and now, 28/4 heads: 1000 tokens 23.8, 14.8, 13.9 us, 8192 73, 54, 48, 131072 898, 764, 692.
 template <bool BF16, bool kInt>
-__global__ void __launch_bounds__(256, 5)
+__global__ void __launch_bounds__(256, 4)
 prep_rows_kernel(QuantRows q, QuantRows k, int q_blocks, const float* partial, const float* mean, int qtype, int half_even, float q_scale) {
   __shared__ float mean_s[128];
   griddep_launch();

@@ -60,6 +60,12 @@ int elementwise_grid(long long work_items, int block) {
   return static_cast<int>(g < 1 ? 1 : (g > cap ? cap : g));
 }
 
+// strided_map_kernel: four 16-byte pieces a thread
+dim3 row_map_grid(int heads, int n, int d) {
+  const long long x = (static_cast<long long>(n) * (d / 8) + 1023) / 1024;
+  return dim3(static_cast<unsigned>(x < 65535 ? x : 65535), heads < 65535 ? heads : 65535);
+}
+
 View4 view_of(const sqattn_tensor& t, int b, int h, int n, int d) {
   View4 v;
   v.ptr = static_cast<const uint8_t*>(t.ptr);
@@ -149,7 +155,7 @@ int launch_prefill(const sqattn_prefill_args* a, const PrefillPlan& pl, cudaStre
   const int64_t cont_v[3] = {static_cast<int64_t>(Hkv) * a->kv_len * D, static_cast<int64_t>(a->kv_len) * D, D};
   if (pl.scale_q) {
     View4 in = view_of(a->q_int8, B, Hq, N, D);
-    const int grid = elementwise_grid(static_cast<long long>(B) * Hq * N * (D / 8), 256);
+    const dim3 grid = row_map_grid(B * Hq, N, D);
     if (bf16) strided_map_kernel<true, 0><<<grid, 256, 0, stream>>>(in, ws + pl.q8_off, scale);
     else strided_map_kernel<false, 0><<<grid, 256, 0, stream>>>(in, ws + pl.q8_off, scale);
     q8 = sqattn_tensor{ws + pl.q8_off, cont_q[0], cont_q[1], cont_q[2]};
@@ -164,7 +170,7 @@ int launch_prefill(const sqattn_prefill_args* a, const PrefillPlan& pl, cudaStre
   }
   if (pl.convert_v) {
     View4 in = view_of(a->v, B, Hkv, a->kv_len, D);
-    const int grid = elementwise_grid(static_cast<long long>(B) * Hkv * a->kv_len * (D / 8), 256);
+    const dim3 grid = row_map_grid(B * Hkv, a->kv_len, D);
     strided_map_kernel<true, 1><<<grid, 256, 0, stream>>>(in, ws + pl.v_off, 1.0f);
     v = sqattn_tensor{ws + pl.v_off, cont_v[0], cont_v[1], cont_v[2]};
   }

@@ -151,6 +151,25 @@ def test_prep_of_slices_equals_the_whole(n, hq, hkv, d):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n,d", [(1, 128), (3, 64), (65, 128), (130, 64)])
+def test_query_rows_bit_for_bit(dtype, n, d):
+    """Rows of very different ranges beside each other (a row's scale comes from one of its lanes), rows of zeros, values that
+    round to a zero of either sign, and quotients on half-integers: the bits of the oracle, on the int8 and the int4 grid."""
+    from longcontext_sqattn_paddle_b200 import ops
+    q, k, v = so.make_inputs(5, 1, n, 4, 2, d, dtype)
+    gen = torch.Generator().manual_seed(n)
+    q *= torch.exp2(torch.randint(-8, 9, (1, n, 4, 1), generator=gen).float()).to(dtype)
+    q[:, :, 1, ::3] *= 2.0 ** -9
+    q[:, ::2, 2] = 0.0
+    q[:, :, 3] = (torch.randint(-254, 255, (1, n, d), generator=gen) / 2).to(dtype)   # a range of 127: halves are ties
+    q[:, :, 3, 0] = 127.0
+    q8, q4, *_ = ops.prep_qkv(q.cuda(), k.cuda(), v.cuda())
+    r8, r4, *_ = so.prep_qkv(q, k, v, 2, "int", "int")
+    for got, want in ((q8, so.scale_q(r8, d)), (q4, so.scale_q(r4, d))):
+        assert torch.equal(got.cpu().view(torch.int16), want.contiguous().view(torch.int16))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_a_nan_in_v_ends_on_the_lowest_step_whatever_lies_beside_it(dtype):
     """The clamp of the integer grid turns a NaN into -128 steps of its channel (the range is taken over the other heads),
     also where none of the channels that one thread holds sits near a half.  The other values are what they are without it."""
