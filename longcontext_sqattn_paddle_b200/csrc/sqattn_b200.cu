@@ -179,10 +179,12 @@ int launch_prefill(const sqattn_prefill_args* a, const PrefillPlan& pl, cudaStre
   CUtensorMap tq8, tq4, tk8, tk4, tv;
   int rc;
   if ((rc = make_tmap_bhnd(&tq8, q8.ptr, a->qk_dtype, q8.stride_b, q8.stride_h, q8.stride_n, B, Hq, N, D, kBlockM, "q_int8"))) return rc;
-  if ((rc = make_tmap_bhnd(&tq4, q4.ptr, a->qk_dtype, q4.stride_b, q4.stride_h, q4.stride_n, B, Hq, N, D, kBlockM, "q_int4"))) return rc;
+  if (alias) tq4 = tq8;
+  else if ((rc = make_tmap_bhnd(&tq4, q4.ptr, a->qk_dtype, q4.stride_b, q4.stride_h, q4.stride_n, B, Hq, N, D, kBlockM, "q_int4"))) return rc;
   if ((rc = make_tmap_bhnd(&tk8, a->k_int8.ptr, a->qk_dtype, a->k_int8.stride_b, a->k_int8.stride_h, a->k_int8.stride_n, B, Hkv, a->kv_len, D, kBlockN, "k_int8"))) return rc;
-  const sqattn_tensor& k4 = alias ? a->k_int8 : a->k_int4;
-  if ((rc = make_tmap_bhnd(&tk4, k4.ptr, a->qk_dtype, k4.stride_b, k4.stride_h, k4.stride_n, B, Hkv, a->kv_len, D, kBlockN, "k_int4"))) return rc;
+  const sqattn_tensor& k4 = a->k_int4;
+  if (alias) tk4 = tk8;
+  else if ((rc = make_tmap_bhnd(&tk4, k4.ptr, a->qk_dtype, k4.stride_b, k4.stride_h, k4.stride_n, B, Hkv, a->kv_len, D, kBlockN, "k_int4"))) return rc;
   if ((rc = make_tmap_bhnd(&tv, v.ptr, SQATTN_F16, v.stride_b, v.stride_h, v.stride_n, B, Hkv, a->kv_len, D, kBlockN, "v"))) return rc;
 
   PrefillParams p;

@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import ctypes as C
 import struct
+from array import array
 from typing import Optional, Sequence
 
 import torch
@@ -47,10 +48,11 @@ def _view(t: torch.Tensor, layout: str) -> L.Tensor:
 
 
 _NO_TENSOR = (0, 0, 0, 0)
-_PREFILL_TENSORS = struct.Struct("25q")   # q_int8, k_int8, q_int4, k_int4, v, o of sqattn_prefill_args, and lse
-assert L.PrefillArgs.lse.offset == _PREFILL_TENSORS.size - 8
-# sqattn_decode_args in the header's order, filled in one call: setting its 45 fields one by one through ctypes took
-# about as long as the launches
+# The argument structs in the header's order, filled in one call each: setting their fields one by one through ctypes took
+# about as long as the launches (a 1000-token call of the operator: 47.3 us field by field, 43.8 like this).
+_PREFILL_ARGS = struct.Struct("4q4q4q4q4q4qq11i4x4q2iqQ6i")
+_PREP_ARGS = struct.Struct("4q4q4q5q10iqQqii")
+assert _PREFILL_ARGS.size == C.sizeof(L.PrefillArgs) and _PREP_ARGS.size == C.sizeof(L.PrepArgs)
 _DECODE_ARGS = struct.Struct("4q4q4q4qq5i4xq6iqQqqqqi4xq")
 assert _DECODE_ARGS.size == C.sizeof(L.DecodeArgs)
 
@@ -111,6 +113,21 @@ def _workspace(nbytes: int, device) -> Optional[torch.Tensor]:
     return ws[off:off + nbytes] if off else ws
 
 
+def _floats(values, count: int) -> array:
+    """``count`` fp32 numbers in host memory; fewer are followed by zeros, more are refused."""
+    x = array("f", map(float, values))
+    if len(x) > count:
+        raise IndexError("invalid index")
+    if len(x) < count:
+        x.extend([0.0] * (count - len(x)))
+    return x
+
+
+def _i32(x) -> int:
+    """The int32 that a C field would hold."""
+    return ((int(x) + 0x80000000) & 0xffffffff) - 0x80000000
+
+
 def prefill(q8, k8, q4, k4, v, *, mode: int, win8=None, win4=None, sink: int = 0, layout: str = "HND",
             out_dtype=torch.float16, return_lse: bool = False, p_fp8_mode: int = 0, q_is_scaled: bool = False,
             out: Optional[torch.Tensor] = None, out_layout: Optional[str] = None, kv_layout: Optional[str] = None,
@@ -130,30 +147,21 @@ def prefill(q8, k8, q4, k4, v, *, mode: int, win8=None, win4=None, sink: int = 0
         out_layout = layout
     lse = torch.empty(b, hq, n, dtype=torch.float32, device=q8.device) if return_lse else None
     qd, kd = _desc(q8, layout), _desc(k8, kv_layout)
-    buf = bytearray(C.sizeof(L.PrefillArgs))
-    _PREFILL_TENSORS.pack_into(buf, 0, *qd, *kd, *(qd if q4 is q8 else _desc(q4, layout)), *(kd if k4 is k8 else _desc(k4, kv_layout)),
-                               *_desc(v, kv_layout), *_desc(out, out_layout), 0 if lse is None else lse.data_ptr())
-    a = L.PrefillArgs.from_buffer(buf)
-    a.q_row_offset, a.head_dim_og = int(q_row_offset), int(head_dim_og)
-    a.q_split_rows, a.q_row_offset2 = int(q_split_rows), int(q_row_offset2)   # second row range of a shard, if any
-    if q_fake_quant is not None:
-        if q_fake_quant not in L.QTYPE:
-            raise ValueError(f"Invalid quantization type: {q_fake_quant}")
-        a.q_fake_quant, a.q_round_half_even = L.QTYPE[q_fake_quant] + 1, int(round_half_even)
-    a.batch, a.num_q_heads, a.num_kv_heads, a.qo_len, a.kv_len, a.head_dim = b, hq, hkv, n, kv_len, d
-    a.qk_dtype, a.v_dtype, a.o_dtype = _dt(q8.dtype), _dt(v.dtype), _dt(out.dtype)
-    a.mode, a.sink_size, a.p_fp8_mode, a.q_is_scaled = mode, int(sink), int(p_fp8_mode), int(q_is_scaled)
-    keep = []
+    if q_fake_quant is not None and q_fake_quant not in L.QTYPE:
+        raise ValueError(f"Invalid quantization type: {q_fake_quant}")
+    windows = (0, 0, 0, 0)
     if mode == L.MODE_RELATIVE_WINDOW:
-        r8 = (C.c_float * hq)(*map(float, win8))
-        r4 = (C.c_float * hq)(*map(float, win4))
-        a.win8_ratios, a.win4_ratios = r8, r4
-        keep += [r8, r4]
+        w8, w4 = _floats(win8, hq), _floats(win4, hq)
+        windows = (w8.buffer_info()[0], w4.buffer_info()[0], 0, 0)
     elif mode == L.MODE_ABSOLUTE_WINDOW:
-        s8 = (C.c_int32 * hq)(*map(int, win8))
-        s4 = (C.c_int32 * hq)(*map(int, win4))
-        a.win8_sizes, a.win4_sizes = s8, s4
-        keep += [s8, s4]
+        w8, w4 = (C.c_int32 * hq)(*map(int, win8)), (C.c_int32 * hq)(*map(int, win4))
+        windows = (0, 0, C.addressof(w8), C.addressof(w4))
+    a = L.PrefillArgs.from_buffer(bytearray(_PREFILL_ARGS.pack(
+        *qd, *kd, *(qd if q4 is q8 else _desc(q4, layout)), *(kd if k4 is k8 else _desc(k4, kv_layout)), *_desc(v, kv_layout),
+        *_desc(out, out_layout), 0 if lse is None else lse.data_ptr(), b, hq, hkv, n, kv_len, d, _dt(q8.dtype), _dt(v.dtype),
+        _dt(out.dtype), mode, _i32(sink), *windows, _i32(p_fp8_mode),
+        int(q_is_scaled), 0, 0, _i32(q_row_offset), _i32(q_split_rows), _i32(q_row_offset2),   # a shard's second row range, if any
+        0 if q_fake_quant is None else L.QTYPE[q_fake_quant] + 1, int(q_fake_quant is not None and round_half_even), _i32(head_dim_og))))
     need = L.lib.sqattn_prefill_workspace_bytes(C.byref(a))
     ws = _workspace(need, q8.device)
     a.workspace, a.workspace_bytes = (ws.data_ptr() if ws is not None else None), need
@@ -179,34 +187,46 @@ def prep_qkv(query, key, value, *, qk_qtype: str = "int", v_qtype: str = "int", 
     b, n, _, d = ref.shape
     dev, dt = ref.device, ref.dtype
     out = out or {}
-    a = L.PrepArgs()
+    parts = 0
     q8 = q4 = k8 = k4 = v8 = None
+    qd = kd = vd = _NO_TENSOR
     hq = hkv = 1
     if query is not None:
         hq = query.shape[2]
-        q8 = out.get("q8") if out.get("q8") is not None else torch.empty(b, hq, n, d, dtype=dt, device=dev)
-        q4 = None if skip_bit4 else (out.get("q4") if out.get("q4") is not None else torch.empty_like(q8))
-        a.q, a.q_bit8, a.q_bit4 = _view(query, "NHD"), q8.data_ptr(), (None if q4 is None else q4.data_ptr())
-        a.parts |= 1
+        q8 = out.get("q8")
+        if q8 is None:
+            q8 = torch.empty((b, hq, n, d), dtype=dt, device=dev)
+        if not skip_bit4:
+            q4 = out.get("q4") if out.get("q4") is not None else torch.empty_like(q8)
+        qd = _desc(query, "NHD")
+        parts |= 1
     if key is not None or value is not None:
-        hkv = (key if key is not None else value).shape[2]
+        kv_in = (key if key is not None else value).shape
+        hkv = kv_in[2]
+        # one length and one set of strides per tensor go down: other shapes would be read past their end
+        if kv_in != (b, n, hkv, d) or (key is not None and value is not None and value.shape != kv_in):
+            raise ValueError(f"query, key and value must be [B, N, H, D] of one batch, length and head_dim, "
+                             f"got {[tuple(t.shape) for t in given]}")
     kv_shape = (b, n, hkv, d) if kv_out_nhd else (b, hkv, n, d)
     if key is not None:
-        k8 = out.get("k8") if out.get("k8") is not None else torch.empty(kv_shape, dtype=dt, device=dev)
-        k4 = None if skip_bit4 else (out.get("k4") if out.get("k4") is not None else torch.empty_like(k8))
-        a.k, a.k_bit8, a.k_bit4 = _view(key, "NHD"), k8.data_ptr(), (None if k4 is None else k4.data_ptr())
-        a.parts |= 2
+        k8 = out.get("k8")
+        if k8 is None:
+            k8 = torch.empty(kv_shape, dtype=dt, device=dev)
+        if not skip_bit4:
+            k4 = out.get("k4") if out.get("k4") is not None else torch.empty_like(k8)
+        kd = _desc(key, "NHD")
+        parts |= 2
     if value is not None:
-        v8 = out.get("v8") if out.get("v8") is not None else torch.empty(kv_shape, dtype=torch.float16, device=dev)
-        a.v, a.v_bit8 = _view(value, "NHD"), v8.data_ptr()
-        a.parts |= 4
-    a.batch, a.num_q_heads, a.num_kv_heads, a.seq_len, a.head_dim = b, hq, hkv, n, d
-    a.dtype, a.qk_qtype, a.v_qtype = _dt(dt), L.QTYPE[qk_qtype], L.QTYPE[v_qtype]
-    a.round_half_even, a.skip_bit4 = int(round_half_even), int(skip_bit4)
-    a.kv_out_nhd = int(kv_out_nhd)
+        v8 = out.get("v8")
+        if v8 is None:
+            v8 = torch.empty(kv_shape, dtype=torch.float16, device=dev)
+        vd = _desc(value, "NHD")
+        parts |= 4
     if k_mean is not None:
         assert k_mean.dtype == torch.float32 and k_mean.is_contiguous() and k_mean.shape == (b, hkv, d)
-        a.k_mean = k_mean.data_ptr()
+    a = L.PrepArgs.from_buffer(bytearray(_PREP_ARGS.pack(
+        *qd, *kd, *vd, *(0 if t is None else t.data_ptr() for t in (q8, q4, k8, k4, v8)), b, hq, hkv, n, d, _dt(dt), L.QTYPE[qk_qtype],
+        L.QTYPE[v_qtype], int(round_half_even), int(skip_bit4), 0, 0, 0 if k_mean is None else k_mean.data_ptr(), int(kv_out_nhd), parts)))
     need = L.lib.sqattn_prep_workspace_bytes(C.byref(a))
     ws = torch.empty(need, dtype=torch.uint8, device=dev)
     a.workspace, a.workspace_bytes = ws.data_ptr(), need
