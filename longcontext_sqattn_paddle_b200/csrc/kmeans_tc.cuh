@@ -515,16 +515,6 @@ __global__ void kmeans_scatter_kernel(const int* idx, const int* slot, const int
         static_cast<int>(i - static_cast<long long>(g) * num_tokens);
   }
 }
-// A 16-bit float as an fp64 whose exponent field is the narrow type's: the value is off by the power of two
-// kNarrowScale, which the fused multiply-add below puts right exactly (zeros and subnormals come out right as well).
-// An integer shift and one DFMA instead of a conversion to fp64, which runs at a quarter of the fp64 rate.
-template <bool BF16>
-__device__ __forceinline__ double narrow_as_double(uint32_t h) {
-  return __hiloint2double(static_cast<int>(((h & 0x7fffu) << (BF16 ? 13 : 10)) | ((h & 0x8000u) << 16)), 0);
-}
-template <bool BF16>
-__device__ __forceinline__ double narrow_scale() { return __hiloint2double(((BF16 ? 896 : 1008) + 1023) << 20, 0); }
-
 // sums[g, c, :] += x[g, t, :] over the members, in fp64 (the caller has zeroed sums).  HBM-bound: one read of x.  The
 // unit of work is kSumRows consecutive entries of the group's member list, NOT a cluster: a warp per cluster left the
 // chip waiting for the warp of the largest one (851 us on average at 8 x 65536 keys in 1024 clusters whose largest held
@@ -557,7 +547,6 @@ kmeans_member_sum_kernel(const uint8_t* x, const int* idx, const int* members, d
     clu[u] = live ? cl[tok[u]] : -1;
   }
   const double scale = narrow_scale<BF16>();
-  constexpr uint32_t kExp = BF16 ? 0x7f807f80u : 0x7c007c00u, kOne = BF16 ? 0x00800080u : 0x04000400u;
   double acc[kPer];
 #pragma unroll
   for (int i = 0; i < kPer; ++i) acc[i] = 0.0;
@@ -596,7 +585,7 @@ kmeans_member_sum_kernel(const uint8_t* x, const int* idx, const int* members, d
         }
         bool special = false;                  // infinities and NaNs have no exponent of their own in the shifted form
 #pragma unroll
-        for (int i = 0; i < kPer / 2; ++i) special |= (((v[q][i] & kExp) + kOne) & 0x80008000u) != 0u;
+        for (int i = 0; i < kPer / 2; ++i) special |= narrow_special<BF16>(v[q][i]);
         if (!special) {
 #pragma unroll
           for (int i = 0; i < kPer / 2; ++i) {

@@ -39,6 +39,22 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// A 16-bit float as an fp64 whose exponent field is the narrow type's: the value is off by the power of two
+// kNarrowScale, which the fused multiply-add below puts right exactly (zeros and subnormals come out right as well).
+// An integer shift and one DFMA instead of a conversion to fp64, which runs at a quarter of the fp64 rate.
+template <bool BF16>
+__device__ __forceinline__ double narrow_as_double(uint32_t h) {
+  return __hiloint2double(static_cast<int>(((h & 0x7fffu) << (BF16 ? 13 : 10)) | ((h & 0x8000u) << 16)), 0);
+}
+template <bool BF16>
+__device__ __forceinline__ double narrow_scale() { return __hiloint2double(((BF16 ? 896 : 1008) + 1023) << 20, 0); }
+// an infinity or a NaN among two 16-bit values: they have no exponent of their own in the shifted form
+template <bool BF16>
+__device__ __forceinline__ bool narrow_special(uint32_t w) {
+  constexpr uint32_t kExp = BF16 ? 0x7f807f80u : 0x7c007c00u, kOne = BF16 ? 0x00800080u : 0x04000400u;
+  return (((w & kExp) + kOne) & 0x80008000u) != 0u;
+}
+
 struct View4 {  // [B,H,N,D] through element strides
   const uint8_t* ptr;
   long long sb, sh, sn;
