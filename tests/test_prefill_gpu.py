@@ -278,3 +278,68 @@ def test_k_mean_override_and_column_sums():
     b = ops.prep_qkv(q.cuda(), k.cuda(), v.cuda(), skip_bit4=True, k_mean=(sums / 777.0).contiguous())
     assert torch.equal(a[0], b[0]) and torch.equal(a[4], b[4])
     assert (a[2].float() != b[2].float()).float().mean().item() < 1e-3
+
+
+# (batch, n, hq, hkv, d, dtype, sink, window ratio, layout): more than 2.9e9 (query, key) pairs in all, from which on long calls
+# take 256-row blocks; odd lengths, a last block of one 128-row tile or less, windows that end inside a 128-key tile, a sink of
+# an odd number of 64-key tiles, all heads of a group apart
+PAIR_CASES = [
+    (12, 2049, 128, 16, 128, torch.bfloat16, None, None, "HND"),
+    (23, 2111, 128, 128, 64, torch.float16, None, None, "NHD"),
+    (10, 4000, 128, 8, 128, torch.bfloat16, 192, 0.096, "NHD"),
+    (8, 4737, 128, 32, 128, torch.float16, 64, 0.11, "HND"),
+    (9, 3265, 128, 16, 128, torch.bfloat16, 0, 0.21, "HND"),
+    (26, 3300, 96, 12, 64, torch.bfloat16, 448, 0.05, "HND"),
+]
+
+
+@pytest.mark.parametrize("batch,n,hq,hkv,d,dtype,sink,ratio,layout", PAIR_CASES)
+def test_long_calls_match_short_ones(batch, n, hq, hkv, d, dtype, sink, ratio, layout):
+    """The same sequences in one call (256-row blocks, 128-key steps) and one by one (128-row blocks, 64-key steps, too little
+    work for the other kernel).  Both hand the tensor core P <= 2^8 rounded to f16 relative to a reference of their own and
+    accumulate in fp32: two results differ by two P roundings (2^-11 each, averaging out over the keys) and two roundings of
+    the output, 2^-8 (bf16) or 2^-11 of the value.  LSE: fp32 sums of the same terms in another order."""
+    from longcontext_sqattn_paddle_b200 import _lib as L, ops
+    g = torch.Generator(device="cuda").manual_seed(n)
+    hnd = layout == "HND"
+    shape = lambda h: (batch, h, n, d) if hnd else (batch, n, h, d)
+    q = torch.randn(shape(hq), generator=g, device="cuda").to(dtype)
+    k = torch.randn(shape(hkv), generator=g, device="cuda").to(dtype)
+    k[..., 3::32] *= 4
+    v = torch.randn(shape(hkv), generator=g, device="cuda").half()
+    if ratio is None:
+        kw = dict(mode=L.MODE_DENSE_CAUSAL)
+    else:
+        w8 = [ratio * (1 + 0.13 * (h % 5)) for h in range(hq)]
+        w4 = [w * (0.5 if h % 3 else 1.0) for h, w in enumerate(w8)]   # an int4 window inside the int8 window is never visited
+        kw = dict(mode=L.MODE_RELATIVE_WINDOW, win8=w8, win4=w4, sink=sink)
+    run = lambda i, j: ops.prefill(q[i:j], k[i:j], q[i:j], k[i:j], v[i:j], layout=layout, out_dtype=dtype, return_lse=True, **kw)
+    whole, lse = run(0, batch)
+    for i in (0, batch - 1):
+        one, lse1 = run(i, i + 1)
+        a, b = whole[i:i + 1].float(), one.float()
+        ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+        assert ((a - b).abs() <= ulp * (a.abs() + b.abs()) + 4 * 2.0 ** -11).all()
+        assert ((a - b).norm() / b.norm()).item() < 1.5 * ulp + 2.0 ** -11
+        assert (lse[i:i + 1] - lse1).abs().max().item() < 1e-4
+    assert torch.isfinite(whole.float()).all()
+
+
+def test_row_ranges_of_a_long_sequence_reproduce_its_rows():
+    """Shards of a sequence that is long enough for 256-row blocks take them too, and give the bits of the whole call, also where
+    a shard's tiles are paired differently (an odd number of 128-row blocks ahead, two ranges in one call)."""
+    from longcontext_sqattn_paddle_b200 import _lib as L, ops
+    n, hq, hkv, d = 20000, 28, 4, 128
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q = torch.randn(1, hq, n, d, generator=g, device="cuda").bfloat16()
+    k = torch.randn(1, hkv, n, d, generator=g, device="cuda").bfloat16()
+    v = torch.randn(1, hkv, n, d, generator=g, device="cuda").half()
+    for kw in (dict(mode=L.MODE_DENSE_CAUSAL), dict(mode=L.MODE_RELATIVE_WINDOW, win8=[0.3] * hq, win4=[0.1] * hq, sink=320)):
+        kw.update(out_dtype=torch.bfloat16, q_is_scaled=True)
+        full = ops.prefill(q, k, q, k, v, **kw)
+        for lo, hi in ((0, 128), (384, 2432), (19968 - 256, n)):
+            part = q[:, :, lo:hi].contiguous()
+            assert torch.equal(ops.prefill(part, k, part.clone(), k.clone(), v, q_row_offset=lo, **kw), full[:, :, lo:hi])
+        rows = torch.cat([q[:, :, 640:1024], q[:, :, 5120:6400]], dim=2).contiguous()
+        part = ops.prefill(rows, k, rows, k, v, q_row_offset=640, q_split_rows=384, q_row_offset2=5120, **kw)
+        assert torch.equal(part, torch.cat([full[:, :, 640:1024], full[:, :, 5120:6400]], dim=2))
