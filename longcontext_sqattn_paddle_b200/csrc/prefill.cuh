@@ -533,19 +533,20 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
         else ok = __all_sync(0xffffffffu, mbar_wait(bar_o_tail + 8, 0, cta_abort, 122));
         if (!ok) break;
         tc_fence_after();
+        const uint64_t al2 = f32x2_pack(alpha, alpha);
 #pragma unroll 1
-        for (int c0 = 0; c0 < D; c0 += 32) {
-          uint32_t o[32];
-          tmem_ld32(tmem + lane_addr + kOCol + c0, o);
-          tmem_wait_ld();
-          const uint64_t al2 = f32x2_pack(alpha, alpha);
+        for (int c0 = 0; c0 < D; c0 += 64) {   // the scores' registers are free: 64 columns at a time, half as many round trips
+          uint32_t o[64];
+          tmem_ld64(tmem + lane_addr + kOCol + c0, o);
+          tmem_wait_ld64(o);
+          uint32_t half[32];
 #pragma unroll
-          for (int c = 0; c < 32; c += 2) {
+          for (int c = 0; c < 64; c += 2) {
             float a, b;
             f32x2_unpack(f32x2_mul(f32x2_pack(__uint_as_float(o[c]), __uint_as_float(o[c + 1])), al2), a, b);
-            o[c] = __float_as_uint(a); o[c + 1] = __float_as_uint(b);
+            half[c & 31] = __float_as_uint(a); half[(c & 31) + 1] = __float_as_uint(b);
+            if ((c & 31) == 30) tmem_st32(tmem + lane_addr + kOCol + c0 + (c & 32), half);
           }
-          tmem_st32(tmem + lane_addr + kOCol + c0, o);
         }
       }
       tmem_wait_st();
