@@ -524,7 +524,12 @@ template <int D, bool BF16>
 int km_member_sums(const uint8_t* x, const int32_t* idx, int32_t groups, int32_t num_tokens, int32_t num_centroids,
                           const KmWorkspace& w, int32_t* counts, double* sums, cudaStream_t stream) {
   const long long gt = static_cast<long long>(groups) * num_tokens, gk = static_cast<long long>(groups) * num_centroids;
-  kmeans_count_kernel<<<elementwise_grid(gt, 256), 256, 0, stream>>>(idx, counts, w.slot, gt, num_tokens, num_centroids);
+  const int count_blocks = (num_tokens + kCountTokens - 1) / kCountTokens;
+  if (num_centroids <= kCountMaxClusters && count_blocks <= 65535)
+    kmeans_count_kernel<<<dim3(groups, count_blocks), kCountThreads, num_centroids * sizeof(int), stream>>>(
+        idx, counts, w.slot, num_tokens, num_centroids);
+  else
+    kmeans_count_many_kernel<<<elementwise_grid(gt, 256), 256, 0, stream>>>(idx, counts, w.slot, gt, num_tokens, num_centroids);
   kmeans_offsets_kernel<<<groups, 1024, 0, stream>>>(counts, w.offsets, num_centroids);
   kmeans_scatter_kernel<<<elementwise_grid(gt, 256), 256, 0, stream>>>(idx, w.slot, w.offsets, w.members, gt, num_tokens, num_centroids);
   SQ_CUDA(cudaMemsetAsync(sums, 0, static_cast<size_t>(gk) * D * sizeof(double), stream));
