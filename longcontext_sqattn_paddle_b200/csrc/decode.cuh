@@ -340,8 +340,8 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           for (int e = 0; e < 4; ++e) { pv[e] = ex2_approx(s[nb][e] - mx[e >> 1]); sum[e >> 1] += pv[e]; }
           uint32_t lo16, hi16;
           if (p.p_fp8) {
-            lo16 = p_fp8_round_f16x2(pv[0], pv[1]);
-            hi16 = p_fp8_round_f16x2(pv[2], pv[3]);
+            lo16 = p_fp8_round_wide_f16x2(pv[0], pv[1]);
+            hi16 = p_fp8_round_wide_f16x2(pv[2], pv[3]);
             if (BF16) {
               // V is bf16, so the tensor-core product takes bf16 operands.  The e4m3-rounded P is an f16 value with
               // up to 11 significant bits: it is split into a bf16 head and a bf16 remainder (exact: at most 3

@@ -244,7 +244,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
     mbar_init(bar_q_empty, 1);
     for (int i = 0; i < KS; ++i) mbar_init(bar_k_full + 8 * i, 1);
     for (int i = 0; i < VS; ++i) mbar_init(bar_v_full + 8 * i, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(bar_s_full + 8 * i, 1); mbar_init(bar_p_full + 8 * i, 128); }
+    for (int i = 0; i < 2; ++i) { mbar_init(bar_s_full + 8 * i, 1); mbar_init(bar_p_full + 8 * i, 4); }
     mbar_init(bar_o_tail, 1);
     mbar_init(bar_o_tail + 8, 1);
     mbar_init(bar_q_ready, 128);
@@ -396,7 +396,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
       // place, with the device functions of the stand-alone preparation kernel (identical bits).  The row's 16-byte
       // chunks sit at chunk ^ (row & 7) inside each 128-byte line of the swizzled tile.
       if (warp == 2 && lane == 0) SQ_STAMP(1, 3);
-      ok = __all_sync(0xffffffffu, mbar_wait(bar_q_full, 0, cta_abort, 124));
+      ok = mbar_wait_warp(bar_q_full, 0, cta_abort, 124);
       if (warp == 2 && lane == 0) SQ_STAMP(1, 15);
       if (ok) {
         uint8_t* qrow = smem + L::kQOff + row_in_tile * 128;
@@ -442,7 +442,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
       const bool fp8 = kFp8 && (flags & kSegFp8);
       const uint32_t s_tmem = tmem + lane_addr + (i & 1) * kBlockN;
       if (warp == 2 && lane == 0) SQ_STAMP(i, 5);
-      ok = __all_sync(0xffffffffu, mbar_wait(bar_s_full + 8 * (i & 1), (i >> 1) & 1, cta_abort, 121));
+      ok = mbar_wait_warp(bar_s_full + 8 * (i & 1), (i >> 1) & 1, cta_abort, 121);
       if (!ok) break;
       tc_fence_after();
       if (warp == 2 && lane == 0) SQ_STAMP(i, 6);
@@ -529,8 +529,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
       if (__any_sync(0xffffffffu, alpha != 1.0f) && i > 0) {
         // P V(i-1) has completed when Q K^T(i+1) has (same issuing thread, in order); the last step waits for the
         // commit that follows P V of the step before it
-        if (i + 1 < nsteps) ok = __all_sync(0xffffffffu, mbar_wait(bar_s_full + 8 * ((i + 1) & 1), ((i + 1) >> 1) & 1, cta_abort, 122));
-        else ok = __all_sync(0xffffffffu, mbar_wait(bar_o_tail + 8, 0, cta_abort, 122));
+        if (i + 1 < nsteps) ok = mbar_wait_warp(bar_s_full + 8 * ((i + 1) & 1), ((i + 1) >> 1) & 1, cta_abort, 122);
+        else ok = mbar_wait_warp(bar_o_tail + 8, 0, cta_abort, 122);
         if (!ok) break;
         tc_fence_after();
         const uint64_t al2 = f32x2_pack(alpha, alpha);
@@ -551,7 +551,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
       }
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(bar_p_full + 8 * (i & 1));
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_p_full + 8 * (i & 1));
       if (warp == 2 && lane == 0) SQ_STAMP(i, 11);
       if (warp == 3 && lane == 0) SQ_STAMP(i, 8);
       if (warp == 4 && lane == 0) SQ_STAMP(i, 10);

@@ -86,8 +86,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return false;
 }
 
-// The same for a converged warp: every lane polls, and the warp agrees on the outcome.
+// The same for a converged warp: every lane polls, and the warp agrees on the outcome.  Most waits are over when they begin:
+// one look and one vote (17 clocks) before the loop, whose branches and vote cost 76 (prefill and calibration 1.3-2.5 % faster;
+// the decode kernel, whose warps wait for memory, 0.5 % slower: it votes on the loop's outcome itself).
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* cta_abort, int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, cta_abort, code));
 }
 
@@ -379,8 +382,25 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
 }
-// (p*448) -> e4m3 (round to nearest even, saturating) -> f16 -> /448 rounded to f16, two values at once.  The division is
-// f16's own: quotient by the reciprocal, exact remainder, one correction.  It is the correctly rounded quotient for each of
+// (p*448) -> e4m3 (round to nearest even, saturating) -> f16 -> /448 rounded to f16, two values at once.
+// v/448 with v an e4m3 value is never within 2^-20 of an f16 rounding boundary (v/7 is either exact
+// or a non-terminating fraction), so multiplying by the fp32 reciprocal and rounding once to f16
+// gives the correctly rounded f16 quotient.  For the decode kernel, whose steps wait for memory: it gains nothing from the
+// shorter form below, and its calls without an FP8 P lose 0.9 % to another allocation of registers.
+__device__ __forceinline__ uint32_t p_fp8_round_wide_f16x2(float lo, float hi) {
+  uint16_t e;
+  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(e) : "f"(hi * 448.0f), "f"(lo * 448.0f));
+  uint32_t h2;
+  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"(e));
+  float flo, fhi;
+  asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %2;\n\tcvt.f32.f16 %0, a;\n\tcvt.f32.f16 %1, b;\n\t}"
+      : "=f"(flo), "=f"(fhi)
+      : "r"(h2));
+  const float inv = 1.0f / 448.0f;
+  return pack_f16x2(flo * inv, fhi * inv);
+}
+
+// The same in f16: quotient by the reciprocal, exact remainder, one correction.  It is the correctly rounded quotient for each of
 // the 127 codes (enumerated, subnormal results among them); five instructions in place of the eight that go through fp32.
 __device__ __forceinline__ uint32_t p_fp8_round_f16x2(float lo, float hi) {
   float l, h;
