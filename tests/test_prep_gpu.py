@@ -188,3 +188,13 @@ def test_a_nan_in_v_ends_on_the_lowest_step_whatever_lies_beside_it(dtype):
     want, got = want.clone(), got.clone()
     want[at] = got[at] = 0.0
     assert torch.equal(want, got)
+
+
+@pytest.mark.parametrize("key_shape,value_shape", [((1, 200, 2, 64), (1, 200, 2, 64)), ((1, 300, 2, 64), (1, 300, 1, 64)),
+                                                   ((1, 300, 2, 128), (1, 300, 2, 128)), ((2, 300, 2, 64), (2, 300, 2, 64))])
+def test_shapes_that_do_not_fit_the_queries_are_refused(key_shape, value_shape):
+    """One length and one head_dim go down for all three tensors: others are refused before anything is launched."""
+    from longcontext_sqattn_paddle_b200 import ops
+    make = lambda shape: torch.zeros(shape, dtype=torch.bfloat16, device="cuda")
+    with pytest.raises(ValueError, match="one batch, length and head_dim"):
+        ops.prep_qkv(make((1, 300, 4, 64)), make(key_shape), make(value_shape))
