@@ -11,7 +11,6 @@
 #include "kmeans_tc.cuh"
 #include "peer_exchange.cuh"
 #include "prefill.cuh"
-#include "prefill_pair.cuh"
 #include "prep.cuh"
 #include "retrieval.cuh"
 #include "window_hist_tc.cuh"
@@ -141,30 +140,6 @@ int plan_prefill(const sqattn_prefill_args* a, PrefillPlan* pl) {
   return SQATTN_OK;
 }
 
-// The rule for prefill_pair_kernel.  It takes an f16 P, prepared queries, and ranges on 64-key boundaries that need the int8
-// operand set alone, i.e. no head whose int4 window reaches further than its int8 window.  It is the faster one where the power
-// limit rules, not the clock: kernels of more than about 1.5 ms, run one after another (28/4 heads, 128-row and 256-row blocks:
-// windows 8192 tokens 185 and 190 us, 20001 734 and 712, 32768 1735 and 1665, 65536 6237 and 5942, 131072 23.6 and 22.6 ms;
-// dense 4000 136 and 141, 16384 1851 and 1802, 32768 7227 and 7043; a lone call of 32768 tokens with windows is 2 % slower).
-// The line is drawn by the work of the whole sequence, so that calls on row ranges of it take the same kernel, whose bits they
-// have to reproduce.
-constexpr double kPairWork = 2.9e9;   // (query, key) pairs over all heads: 1.5 TFLOP at D = 128
-bool pair_fits(const PrefillParams& p, int d) {
-  if (p.p_fp8_mode || p.q_fake_quant || p.mode == SQATTN_MODE_ABSOLUTE_WINDOW) return false;
-  const double n = p.n_total;
-  double pairs = 0;
-  for (int h = 0; h < p.hq; ++h) {
-    double seen = n / 2;
-    if (p.mode == SQATTN_MODE_RELATIVE_WINDOW) {
-      if (p.w4[h] > p.w8[h]) return false;
-      const double window = static_cast<double>(p.sink) + (p.w8[h] > 64 ? p.w8[h] : 64);
-      seen = window < seen ? window : seen;
-    }
-    pairs += n * seen;
-  }
-  return pairs * p.batch * (d / 128.0) >= kPairWork;
-}
-
 template <int D>
 int launch_prefill(const sqattn_prefill_args* a, const PrefillPlan& pl, cudaStream_t stream, float* dump,
                    long long* dump_t = nullptr, float* dump_p = nullptr) {
@@ -234,17 +209,6 @@ int launch_prefill(const sqattn_prefill_args* a, const PrefillPlan& pl, cudaStre
   }
   const long long grid = static_cast<long long>(p.nblk) * Hq * B;
   if (grid > 0x7fffffffll) return fail(SQATTN_ERR_UNSUPPORTED, "grid too large");
-  if (!dump && !dump_t && !dump_p && pair_fits(p, D)) {
-    using L = PairSmem<D>;
-    CUtensorMap tk, tvp;   // tiles of 128 keys
-    if ((rc = make_tmap_bhnd(&tk, a->k_int8.ptr, a->qk_dtype, a->k_int8.stride_b, a->k_int8.stride_h, a->k_int8.stride_n, B, Hkv, a->kv_len, D, kPairN, "k_int8"))) return rc;
-    if ((rc = make_tmap_bhnd(&tvp, v.ptr, SQATTN_F16, v.stride_b, v.stride_h, v.stride_n, B, Hkv, a->kv_len, D, kPairN, "v"))) return rc;
-    const int items = PairGrid(p).items();
-    auto kernel = prefill_pair_kernel<D>;
-    SQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynBytes));
-    SQ_CUDA(launch_overlapped(4, kernel, dim3(items < 148 ? items : 148), dim3(kPairThreads), L::kDynBytes, stream, tq8, tk, tvp, p));
-    return SQATTN_OK;
-  }
 #define SQ_LAUNCH_PREFILL(DUMP, FP8)                                                                                     \
   do {                                                                                                                   \
     using L = PrefillSmem<D, 2, 3>;   /* two K stages (tied to the two S buffers), three V stages, two CTAs per SM */    \

@@ -280,25 +280,28 @@ def test_k_mean_override_and_column_sums():
     assert (a[2].float() != b[2].float()).float().mean().item() < 1e-3
 
 
-# (batch, n, hq, hkv, d, dtype, sink, window ratio, layout): more than 2.9e9 (query, key) pairs in all, from which on long calls
-# take 256-row blocks; odd lengths, a last block of one 128-row tile or less, windows that end inside a 128-key tile, a sink of
-# an odd number of 64-key tiles, all heads of a group apart
-PAIR_CASES = [
+# (batch, n, hq, hkv, d, dtype, sink, window ratio, layout): 1.5 TFLOP and more in the whole call; odd lengths, a last block of one
+# 128-row tile or less, windows that end inside a pair of 64-key tiles, a sink of an odd number of them, all heads of a group apart
+WHOLE_CASES = [
     (12, 2049, 128, 16, 128, torch.bfloat16, None, None, "HND"),
     (23, 2111, 128, 128, 64, torch.float16, None, None, "NHD"),
     (10, 4000, 128, 8, 128, torch.bfloat16, 192, 0.096, "NHD"),
     (8, 4737, 128, 32, 128, torch.float16, 64, 0.11, "HND"),
     (9, 3265, 128, 16, 128, torch.bfloat16, 0, 0.21, "HND"),
-    (26, 3300, 96, 12, 64, torch.bfloat16, 448, 0.05, "HND"),
+    (30, 3300, 96, 12, 64, torch.bfloat16, 448, 0.06, "HND"),
 ]
 
 
-@pytest.mark.parametrize("batch,n,hq,hkv,d,dtype,sink,ratio,layout", PAIR_CASES)
-def test_long_calls_match_short_ones(batch, n, hq, hkv, d, dtype, sink, ratio, layout):
-    """The same sequences in one call (256-row blocks, 128-key steps) and one by one (128-row blocks, 64-key steps, too little
-    work for the other kernel).  Both hand the tensor core P <= 2^8 rounded to f16 relative to a reference of their own and
-    accumulate in fp32: two results differ by two P roundings (2^-11 each, averaging out over the keys) and two roundings of
-    the output, 2^-8 (bf16) or 2^-11 of the value.  LSE: fp32 sums of the same terms in another order."""
+def _same_bits(a, b):
+    as_int = lambda t: t.contiguous().view(torch.int32 if t.dtype == torch.float32 else torch.int16)
+    return torch.equal(as_int(a), as_int(b))
+
+
+@pytest.mark.parametrize("batch,n,hq,hkv,d,dtype,sink,ratio,layout", WHOLE_CASES)
+def test_a_sequence_has_the_same_bits_alone_in_a_batch_and_by_heads(batch, n, hq, hkv, d, dtype, sink, ratio, layout):
+    """How much work a call has decides nothing about a row's result: the sequences of a large call, one of them alone, and one
+    KV head's query heads alone give the same bits, an infinite query element (a row whose first scores are all -inf) and scores
+    that climb by octaves along the keys included."""
     from longcontext_sqattn_paddle_b200 import _lib as L, ops
     g = torch.Generator(device="cuda").manual_seed(n)
     hnd = layout == "HND"
@@ -307,27 +310,52 @@ def test_long_calls_match_short_ones(batch, n, hq, hkv, d, dtype, sink, ratio, l
     k = torch.randn(shape(hkv), generator=g, device="cuda").to(dtype)
     k[..., 3::32] *= 4
     v = torch.randn(shape(hkv), generator=g, device="cuda").half()
-    if ratio is None:
+    # the last sequence's scores climb along the keys, for every third query row: one channel of K grows, that of Q is constant
+    ramp = (torch.arange(n, device="cuda") / 24 + 20 * torch.rand(n, generator=g, device="cuda")).to(dtype)
+    k[-1, ..., 0] = ramp if hnd else ramp[:, None]
+    rows = torch.arange(n, device="cuda") % 3 == 0
+    q[-1, ..., 0] = (rows if hnd else rows[:, None]).to(dtype) * d ** 0.5 / 1.4427
+    q[:, 0, 0, 7] = float("inf")
+    k[:, 0, 0, 7] = -1.0
+
+    def run(i, j, h0=0, h1=hkv):
+        groups = hq // hkv
+        cut = (lambda t, a, b: t[i:j, a:b].contiguous()) if hnd else (lambda t, a, b: t[i:j, :, a:b].contiguous())
         kw = dict(mode=L.MODE_DENSE_CAUSAL)
-    else:
-        w8 = [ratio * (1 + 0.13 * (h % 5)) for h in range(hq)]
-        w4 = [w * (0.5 if h % 3 else 1.0) for h, w in enumerate(w8)]   # an int4 window inside the int8 window is never visited
-        kw = dict(mode=L.MODE_RELATIVE_WINDOW, win8=w8, win4=w4, sink=sink)
-    run = lambda i, j: ops.prefill(q[i:j], k[i:j], q[i:j], k[i:j], v[i:j], layout=layout, out_dtype=dtype, return_lse=True, **kw)
+        if ratio is not None:
+            w8 = [ratio * (1 + 0.13 * (h % 5)) for h in range(hq)][h0 * groups:h1 * groups]
+            w4 = [w * (0.5 if h % 3 else 1.0) for h, w in enumerate(w8)]   # an int4 window inside the int8 window is never visited
+            kw = dict(mode=L.MODE_RELATIVE_WINDOW, win8=w8, win4=w4, sink=sink)
+        qc, kc, vc = cut(q, h0 * groups, h1 * groups), cut(k, h0, h1), cut(v, h0, h1)
+        return ops.prefill(qc, kc, qc, kc, vc, layout=layout, out_dtype=dtype, return_lse=True, **kw)
+
     whole, lse = run(0, batch)
     for i in (0, batch - 1):
         one, lse1 = run(i, i + 1)
-        a, b = whole[i:i + 1].float(), one.float()
-        ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
-        assert ((a - b).abs() <= ulp * (a.abs() + b.abs()) + 4 * 2.0 ** -11).all()
-        assert ((a - b).norm() / b.norm()).item() < 1.5 * ulp + 2.0 ** -11
-        assert (lse[i:i + 1] - lse1).abs().max().item() < 1e-4
-    assert torch.isfinite(whole.float()).all()
+        assert _same_bits(whole[i:i + 1], one) and _same_bits(lse[i:i + 1], lse1)
+    groups = hq // hkv
+    for i in (0, batch - 1):
+        some, lse1 = run(i, i + 1, hkv - 1, hkv)
+        w = whole[i:i + 1]
+        assert _same_bits(w[:, -groups:] if hnd else w[:, :, -groups:], some) and _same_bits(lse[i:i + 1, -groups:], lse1)
+    assert whole[:, 0, 0].isnan().all() and torch.isfinite(whole[:, -1, -1]).all()
+
+
+def test_raw_queries_of_a_long_call_match_prepared_ones():
+    """A call that fake-quantises its queries itself reproduces the one on prepared queries bit for bit, whatever its length."""
+    from longcontext_sqattn_paddle_b200 import _lib as L, ops
+    n, hq, hkv, d = 33000, 28, 4, 128
+    q, k, v = so.make_inputs(17, 1, n, hq, hkv, d, torch.bfloat16)
+    q, k, v = q.cuda(), k.cuda(), v.cuda()
+    q8, _, k8, _, v8 = ops.prep_qkv(q, k, v, skip_bit4=True)
+    kw = dict(mode=L.MODE_RELATIVE_WINDOW, win8=[0.12] * hq, win4=[0.1] * hq, sink=256, out_dtype=torch.bfloat16, return_lse=True)
+    a, la = ops.prefill(q8, k8, q8, k8, v8, q_is_scaled=True, **kw)
+    b, lb = ops.prefill(q, k8, q, k8, v8, layout="NHD", kv_layout="HND", q_fake_quant="int", **kw)
+    assert _same_bits(a, b.transpose(1, 2)) and _same_bits(la, lb)
 
 
 def test_row_ranges_of_a_long_sequence_reproduce_its_rows():
-    """Shards of a sequence that is long enough for 256-row blocks take them too, and give the bits of the whole call, also where
-    a shard's tiles are paired differently (an odd number of 128-row blocks ahead, two ranges in one call)."""
+    """Shards of a long sequence give the bits of the whole call: an odd number of 128-row blocks ahead, two ranges in one call."""
     from longcontext_sqattn_paddle_b200 import _lib as L, ops
     n, hq, hkv, d = 20000, 28, 4, 128
     g = torch.Generator(device="cuda").manual_seed(3)
