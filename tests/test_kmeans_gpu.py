@@ -212,3 +212,57 @@ def test_member_lists_with_fewer_ranges_than_usual(g, t, k):
     for b in range(g):
         order = torch.sort(idx[b].long(), stable=True).indices          # members one cluster after another, in token order
         assert torch.equal(lists[b][torch.arange(lists.shape[2]) < n[b][:, None]], order)
+
+
+def _exact_assignment(data, cent):
+    """Largest fp64 score, lowest index on ties; a score that is not a number is never taken, 0 where none is left."""
+    score = data.double() @ cent.double().transpose(1, 2)
+    score = score.nan_to_num(nan=-float("inf"), posinf=float("inf"), neginf=-float("inf"))
+    best = score.amax(-1, keepdim=True)
+    k = cent.shape[1]
+    return torch.where(score == best, torch.arange(k, device=data.device), k).amin(-1)
+
+
+@pytest.mark.parametrize("g,t,k,d,twice,zeros", [
+    (2, 10000, 6144, 128, 64, 0), (1, 20000, 6176, 128, 64, 0), (2, 7000, 9600, 64, 4800, 0), (1, 10000, 12320, 128, 64, 0),
+    (1, 5000, 24608, 128, 12304, 0), (1, 2500, 49152, 64, 64, 0), (1, 900, 12320, 128, 6160, 0), (2, 9000, 64, 128, 32, 4500),
+    (8, 30000, 64, 64, 8, 0), (8, 250, 1024, 128, 8, 0)])
+def test_many_centroids_and_long_lists(g, t, k, d, twice, zeros):
+    """Every number of tokens that a sweep of the re-scoring takes (8, 4, 2 and 1 as their scores' memory allows, 1 in small
+    calls), up to the most centroids a group may have; ranks counted by CTAs and, above 8192 clusters, by warps; and more listed
+    tokens than the list holds.  ``twice`` centroids are there twice: their tokens are re-scored, and the lower index wins.
+    Exact indices, counts and sums."""
+    from longcontext_sqattn_paddle_b200.cache_hub import kmeans as km
+    gen = torch.Generator(device="cuda").manual_seed(k + t)
+    data = torch.randn(g, t, d, generator=gen, device="cuda").bfloat16()
+    data[:, t - zeros:] = 0.0
+    cent = torch.randn(g, k, d, generator=gen, device="cuda").bfloat16()
+    cent[:, k - twice:] = cent[:, :twice]
+    want = _exact_assignment(data, cent)
+    want = torch.where(want >= k - twice, want - (k - twice), want)
+    new, idx, counts = km.k_means_train(data, cent.clone(), False)
+    assert torch.equal(idx.long(), want)
+    n = torch.stack([torch.bincount(r, minlength=k) for r in want])
+    assert torch.equal(counts.long(), n)
+    sums = torch.zeros(g, k, d, dtype=torch.float64, device="cuda").scatter_add_(1, want[..., None].expand(-1, -1, d), data.double())
+    mean = torch.where(n[..., None] > 0, (sums.float() / n[..., None].float()).bfloat16(), cent)
+    assert torch.equal(new, mean)
+    assert torch.equal(km.index_add(data, idx, k), sums.float().bfloat16())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("t,k,d", [(300, 32, 128), (700, 64, 64), (2000, 416, 128)])
+def test_assignment_with_infinities_and_nans(dtype, t, k, d):
+    """Infinite and NaN elements in keys, then in centroids: the largest score that is a number, whatever stands beside it."""
+    from longcontext_sqattn_paddle_b200.cache_hub import kmeans as km
+    gen = torch.Generator(device="cuda").manual_seed(t)
+    data = torch.randn(2, t, d, generator=gen, device="cuda").to(dtype)
+    cent = torch.randn(2, k, d, generator=gen, device="cuda").to(dtype)
+    odd = data.clone()
+    odd[:, 3::7, 1], odd[:, 5::11, 2], odd[:, 4::13, 0] = float("inf"), -float("inf"), float("nan")
+    wild = cent.clone()
+    wild[0, 3, :] = float("nan")
+    wild[0, 7, 3], wild[0, 9, 4], wild[1, k - 1, 5] = float("inf"), -float("inf"), float("nan")
+    for x, c in ((odd, cent), (data, wild), (odd, wild)):
+        _, idx, _ = km.k_means_train(x, c.clone(), False)
+        assert torch.equal(idx.long(), _exact_assignment(x, c))
