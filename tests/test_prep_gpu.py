@@ -170,6 +170,26 @@ def test_query_rows_bit_for_bit(dtype, n, d):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("qtype", ["e4m3", "e5m2"])
+@pytest.mark.parametrize("n,d", [(1, 128), (3, 64), (65, 128), (130, 64)])
+def test_emulated_float_rows_do_not_depend_on_their_place(dtype, qtype, n, d):
+    """A thread takes its four rows one after another: a row's bits are those of the same row in another place, beside rows of
+    other ranges and rows of zeros, on both outputs."""
+    from longcontext_sqattn_paddle_b200 import ops
+    q, *_ = so.make_inputs(6, 1, n, 4, 2, d, dtype)
+    q *= torch.exp2(torch.randint(-8, 9, (1, n, 4, 1), generator=torch.Generator().manual_seed(n)).float()).to(dtype)
+    q[:, ::2, 2] = 0.0
+    q = q.cuda()
+    whole = ops.prep_qkv(q, None, None, qk_qtype=qtype)[:2]
+    bits = lambda t: t.contiguous().view(torch.int16)
+    for shift in (1, 8, 16, n // 2):
+        moved = ops.prep_qkv(q.roll(shift, 1), None, None, qk_qtype=qtype)[:2]
+        assert all(torch.equal(bits(a.roll(shift, 2)), bits(b)) for a, b in zip(whole, moved))
+    alone = ops.prep_qkv(q[:, n - 1:], None, None, qk_qtype=qtype)[:2]
+    assert all(torch.equal(bits(a[:, :, n - 1:]), bits(b)) for a, b in zip(whole, alone))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_a_nan_in_v_ends_on_the_lowest_step_whatever_lies_beside_it(dtype):
     """The clamp of the integer grid turns a NaN into -128 steps of its channel (the range is taken over the other heads),
     also where none of the channels that one thread holds sits near a half.  The other values are what they are without it."""
