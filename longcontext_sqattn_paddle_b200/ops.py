@@ -173,8 +173,8 @@ def prep_qkv(query, key, value, *, qk_qtype: str = "int", v_qtype: str = "int", 
              skip_bit4: bool = False, k_mean: Optional[torch.Tensor] = None, kv_out_nhd: bool = False,
              out: Optional[dict] = None):
     """sqattn_prep_qkv: NHD inputs -> (q_bit8, q_bit4, k_bit8, k_bit4, v_bit8) contiguous HND; q pre-scaled,
-    K/V with their own Hkv heads, v_bit8 in fp16.  k_mean [B,Hkv,D] fp32 overrides the sequence mean of K;
-    kv_out_nhd writes the K/V outputs token-major [B,N,Hkv,D].  Any of query/key/value may be None: only the
+    K/V with their own Hkv heads, v_bit8 in fp16; of longer keys and values the first N rows are prepared.
+    k_mean [B,Hkv,D] fp32 overrides the sequence mean of K; kv_out_nhd writes the K/V outputs token-major [B,N,Hkv,D].  Any of query/key/value may be None: only the
     tensors given are prepared (their outputs are returned, the others are None).  ``out`` may hold
     preallocated outputs under the keys q8, q4, k8, k4, v8."""
     given = [t for t in (query, key, value) if t is not None]
@@ -201,12 +201,12 @@ def prep_qkv(query, key, value, *, qk_qtype: str = "int", v_qtype: str = "int", 
         qd = _desc(query, "NHD")
         parts |= 1
     if key is not None or value is not None:
-        kv_in = (key if key is not None else value).shape
-        hkv = kv_in[2]
-        # one length and one set of strides per tensor go down: other shapes would be read past their end
-        if kv_in != (b, n, hkv, d) or (key is not None and value is not None and value.shape != kv_in):
-            raise ValueError(f"query, key and value must be [B, N, H, D] of one batch, length and head_dim, "
-                             f"got {[tuple(t.shape) for t in given]}")
+        hkv = (key if key is not None else value).shape[2]
+        # one length, one count of KV heads and one set of strides per tensor go down: shorter ones would be read past their end
+        for t in (key, value):
+            if t is not None and (t.shape[0] != b or t.shape[1] < n or t.shape[2] < hkv or t.shape[3] != d):
+                raise ValueError(f"query, key and value must be [B, N, H, D] of one batch, length and head_dim (keys and values "
+                                 f"beyond the first's length are left out), got {[tuple(t.shape) for t in given]}")
     kv_shape = (b, n, hkv, d) if kv_out_nhd else (b, hkv, n, d)
     if key is not None:
         k8 = out.get("k8")

@@ -218,3 +218,15 @@ def test_shapes_that_do_not_fit_the_queries_are_refused(key_shape, value_shape):
     make = lambda shape: torch.zeros(shape, dtype=torch.bfloat16, device="cuda")
     with pytest.raises(ValueError, match="one batch, length and head_dim"):
         ops.prep_qkv(make((1, 300, 4, 64)), make(key_shape), make(value_shape))
+
+
+@pytest.mark.parametrize("keys,values,value_heads", [(300, 300, 2), (301, 300, 2), (300, 452, 2), (1000, 600, 3)])
+def test_of_longer_keys_and_values_the_first_rows_are_prepared(keys, values, value_heads):
+    """Keys and values that reach beyond the queries (a cache with room, a chunk's queries) are prepared up to the queries' length."""
+    from longcontext_sqattn_paddle_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(keys + values)
+    make = lambda n, h: torch.randn(1, n, h, 128, generator=gen, device="cuda").bfloat16()
+    q, k, v = make(300, 4), make(keys, 2), make(values, value_heads)
+    got, want = ops.prep_qkv(q, k, v), ops.prep_qkv(q, k[:, :300], v[:, :300, :2])
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert torch.equal(ops.prep_qkv(None, k[:, :300], v)[4], want[4])
