@@ -60,9 +60,12 @@ int elementwise_grid(long long work_items, int block) {
   return static_cast<int>(g < 1 ? 1 : (g > cap ? cap : g));
 }
 
-// strided_map_kernel: four 16-byte pieces a thread
+// strided_map_kernel: four 16-byte pieces a thread, one where four leave less than two blocks to an SM (dense calls, scaled copy of
+// Q and f16 copy of V ahead of them, 28/4 heads, four and by this rule: 500 tokens 19.8 and 19.1 us, 1000 28.8 and 28.1; one
+// piece everywhere: 1500 tokens 42.8 and 41.4, 3000 93.0 and 90.1).
 dim3 row_map_grid(int heads, int n, int d) {
-  const long long x = (static_cast<long long>(n) * (d / 8) + 1023) / 1024;
+  const long long pieces = static_cast<long long>(n) * (d / 8), four = (pieces + 1023) / 1024;
+  const long long x = four * heads < 2 * 148 ? (pieces + 255) / 256 : four;
   return dim3(static_cast<unsigned>(x < 65535 ? x : 65535), heads < 65535 ? heads : 65535);
 }
 

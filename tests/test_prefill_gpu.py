@@ -371,3 +371,20 @@ def test_row_ranges_of_a_long_sequence_reproduce_its_rows():
         rows = torch.cat([q[:, :, 640:1024], q[:, :, 5120:6400]], dim=2).contiguous()
         part = ops.prefill(rows, k, rows, k, v, q_row_offset=640, q_split_rows=384, q_row_offset2=5120, **kw)
         assert torch.equal(part, torch.cat([full[:, :, 640:1024], full[:, :, 5120:6400]], dim=2))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n,d", [(1, 128), (640, 128), (641, 128), (1280, 64), (1281, 64)])
+def test_copies_ahead_of_the_kernel(dtype, n, d):
+    """The scaled copy of Q and the f16 copy of V on either side of the line between one and four 16-byte pieces a thread, out of
+    strided views: the bits of a call that gets both ready-made."""
+    from longcontext_sqattn_paddle_b200 import _lib as L, ops
+    hq, hkv = 28, 4
+    g = torch.Generator(device="cuda").manual_seed(n)
+    qkv = torch.randn(2, n, (hq + 2 * hkv) * d, generator=g, device="cuda").to(dtype)
+    q, k, v = (t.view(2, n, -1, d) for t in qkv.split([hq * d, hkv * d, hkv * d], dim=-1))
+    kw = dict(mode=L.MODE_DENSE_CAUSAL, layout="NHD", out_dtype=dtype, return_lse=True)
+    o, lse = ops.prefill(q, k, q, k, v, **kw)
+    scaled = so.scale_q(q.cpu(), d).cuda()
+    want, want_lse = ops.prefill(scaled, k, scaled, k, v.half(), q_is_scaled=True, **kw)
+    assert _same_bits(o, want) and _same_bits(lse, want_lse)

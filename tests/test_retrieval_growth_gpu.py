@@ -141,3 +141,22 @@ def test_selection_at_the_crossing_score(k, d, kind):
                                              heads, k, d, width, total, budget, out.data_ptr(), cnt.data_ptr(), total, total, _stream()))
         for gi, sel in enumerate(ko.select_clusters(qm, cent, size, lists, budget)):
             assert cnt[gi].item() == len(sel) and torch.equal(out[gi, :len(sel)].cpu(), sel)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("d", [64, 128])
+def test_selection_with_infinite_and_nan_centroids(dtype, d):
+    """Centroid elements without an exponent of their own (infinities, NaNs), subnormals and zeros: the clusters that the oracle
+    takes (a NaN score last)."""
+    from longcontext_sqattn_paddle_b200.cache_hub import ClusteredKV
+    hkv, hq, n, budget, cap = 2, 8, 6000, 1500, 4096
+    cache = ClusteredKV(_data(hkv, n, d, 4, dtype).cuda(), _data(hkv, n, d, 5, dtype).cuda(), num_iters=3)
+    q = torch.randn(hq, d, generator=torch.Generator().manual_seed(6)).to(dtype)
+    qm = _mean_query(q, hkv)
+    c = cache.centroids
+    c[:, 2, 3], c[:, 4, 5], c[:, 11, 1] = float("nan"), float("inf"), -float("inf")
+    c[:, 9], c[:, 12], c[:, 13, 7] = 0.0, c[:, 12] * 2.0 ** (-14 if dtype == torch.float16 else -126), -0.0
+    idx, count = cache.select(q.cuda(), budget, cap)
+    sel = ko.select_clusters(qm, c.cpu(), cache.cluster_size.cpu(), cache.clusters.cpu(), budget)
+    for h in range(hkv):
+        assert torch.equal(idx[h, :int(count[h])].cpu(), sel[h])
