@@ -201,10 +201,11 @@ def prep_qkv(query, key, value, *, qk_qtype: str = "int", v_qtype: str = "int", 
         qd = _desc(query, "NHD")
         parts |= 1
     if key is not None or value is not None:
-        hkv = (key if key is not None else value).shape[2]
+        kv_in = (key if key is not None else value).shape
+        hkv = kv_in[2]
         # one length, one count of KV heads and one set of strides per tensor go down: shorter ones would be read past their end
-        for t in (key, value):
-            if t is not None and (t.shape[0] != b or t.shape[1] < n or t.shape[2] < hkv or t.shape[3] != d):
+        if kv_in != (b, n, hkv, d) or (key is not None and value is not None and value.shape != kv_in):
+            if any(t.shape[0] != b or t.shape[1] < n or t.shape[2] < hkv or t.shape[3] != d for t in (key, value) if t is not None):
                 raise ValueError(f"query, key and value must be [B, N, H, D] of one batch, length and head_dim (keys and values "
                                  f"beyond the first's length are left out), got {[tuple(t.shape) for t in given]}")
     kv_shape = (b, n, hkv, d) if kv_out_nhd else (b, hkv, n, d)
