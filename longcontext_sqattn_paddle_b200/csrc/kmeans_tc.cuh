@@ -313,12 +313,14 @@ kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tm_data, const __gri
   }
 }
 
-// Exact re-scoring of the listed tokens, up to kRecheckTokens consecutive ones of the list per CTA and sweep (the CTAs loop
-// over the list; neighbours in it mostly belong to one group, and a sweep serves those of one group):
+// Exact re-scoring of the listed tokens, per_sweep consecutive ones of the list per CTA (the CTAs loop over the list).  A sweep
+// serves those of one group; neighbours in a long list mostly belong to one, in a short one to several (the rule is at the launch):
 //   1. fp32 scores of ALL centroids of the group into shared memory: mma.sync m16n8k16 with 16 centroid rows as A, straight
 //      from global memory (16 bytes of a row per lane; the order of the channels inside a product does not matter), and the
 //      tokens as the columns of B.  A token's own sweep with fp32 FMAs took 15 instructions per row for unpacking and shuffles
-//      and one read of all centroids per token: 74 us for the 1600 or so tokens of an iteration (8 x 65536 keys, 1024 centroids), 33 us like this: latency of a sweep and of the fp64 chain;
+//      and one read of all centroids per token: 42-86 us for the tokens of an iteration (8 x 65536 keys, 1024 centroids), 30-32 us
+//      like this, the latency of a sweep and of the fp64 chain; 4 x 262144 keys, 4096 centroids 400-950 and 153-302, 2 x 1048576,
+//      16384 (two tokens a sweep) 4760-17800 and 3280-11770;
 //   2. a warp per token: the candidates, i.e. centroids whose fp32 score lies within the error band of the largest one (the
 //      same bound as in the assignment kernel, which also covers this pass's own rounding); a score that is not a number counts;
 //   3. the candidates' exact scores in fp64 (exact products, index-order sum), the largest wins, the lowest index
@@ -343,7 +345,7 @@ __device__ __forceinline__ double exact_score(const double* kd, const uint8_t* r
   return s;
 }
 
-// per_sweep <= kRecheckTokens: as many tokens as the scores' shared memory holds
+// per_sweep <= kRecheckTokens, at most as many tokens as the scores' shared memory holds
 template <int D, bool BF16>
 __global__ void __launch_bounds__(256)
 kmeans_recheck_list_kernel(const uint8_t* data, const uint8_t* cent, int* idx, const int* flagged, const int* flagged_count,

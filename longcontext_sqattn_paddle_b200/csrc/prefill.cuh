@@ -309,9 +309,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant_
     // The whole warp runs this loop converged and one elected lane issues each instruction: written as
     // `if (lane == 0) { ... }` the descriptors and addresses are per-thread values for the compiler and one
     // tcgen05.mma cost the issuing thread ~107 cycles (a commit ~350), 1200 cycles for the 8 MMAs and the commit
-    // of a Q K^T against ~540 now (clock stamps of a debug build).  An N = 64 instruction takes 48
-    // clocks (the bandwidth of shared memory), an N = 128 one 64.  There is ONE commit per step, behind Q K^T; since one thread's MMAs complete in
-    // issue order that commit also reports P V of two steps earlier, which is all the other warps need to know.
+    // of a Q K^T against ~540 now (clock stamps of a debug build).  An N = 64 instruction takes 48 clocks (the
+    // bandwidth of shared memory), an N = 128 one 64.  There is ONE commit per step, behind Q K^T; since one
+    // thread's MMAs complete in issue order that commit also reports P V of two steps earlier, which is all the
+    // other warps need to know.
     // Issue order QK(i+1), PV(i): S buffer (i+1)&1 still holds P(i-1), which PV(i-1), issued earlier by this
     // same thread, consumes first (the tensor pipe executes one thread's MMAs in issue order).
     {

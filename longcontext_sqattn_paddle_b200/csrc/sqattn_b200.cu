@@ -520,6 +520,7 @@ int km_launch_assign(const void* data, const void* centroids, int32_t dtype, int
   p.flagged_cap = w.flagged_cap; p.max_cnorm2 = w.max_cnorm2; p.groups = groups; p.num_tokens = num_tokens; p.num_centroids = num_centroids;
   p.bf16 = dtype == SQATTN_BF16;
   using L = KmeansTcSmem<D>;
+  static_assert(L::kTotal <= 227 * 1024, "shared memory of a CTA");
   SQ_CUDA(cudaFuncSetAttribute(kmeans_assign_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
   const long long items = static_cast<long long>(groups) * ((num_tokens + kKtTokens - 1) / kKtTokens);
   const unsigned grid = static_cast<unsigned>(items < 148 ? items : 148);   // persistent: one CTA per SM
