@@ -826,13 +826,13 @@ int sqattn_kmeans_assign(const void* data, const void* centroids, int32_t dtype,
                             : km_launch_assign<64>(data, centroids, dtype, groups, num_tokens, num_centroids, idx, w, stream)))
     return rc;
   {
-    // Neighbours in the list often belong to different groups, which a sweep takes one after another: a token for itself where
-    // the usual list (0.25 % of the tokens) leaves no CTA more than one, or few enough for their own sweeps.  A Lloyd iteration,
-    // eight and one: 8 x 4000 keys, 64 centroids 58.1 and 42.5 us, 8 x 16000, 256 71.0 and 63.2, 8 x 29000, 448 112.9 and 108.1,
-    // 4 x 50000, 768 120.8 and 122.3.  The fp32 scores of a sweep's tokens: 192 KB at most.
-    constexpr int kGrid = 148 * 4;
-    const long long sweeps = static_cast<long long>(groups) * num_tokens * (num_centroids > 512 ? num_centroids : 512);
-    int per_sweep = sweeps <= 400ll * kGrid * 512 ? 1 : kRecheckTokens;
+    // Neighbours in the list often belong to different groups, which a sweep takes one after another: a token for itself where the
+    // list (0.25 % of the tokens as a rule) is short or its sweeps are.  A Lloyd iteration, eight and one: 8 x 256 keys, 1024
+    // centroids 113 and 67 us, 8 x 4000, 64 57.7 and 42.1, 8 x 24000, 384 93.9 and 87.2, 512 x 1024, 32 151 and 134; on the other
+    // side of the line 8 x 65536, 192 135.2 and 137.0, 4 x 50000, 768 120.8 and 122.3.  The fp32 scores of a sweep's tokens: 192
+    // KB at most.
+    const long long sweeps = static_cast<long long>(groups) * num_tokens * (num_centroids > 128 ? num_centroids : 128);
+    int per_sweep = sweeps <= 100000000ll ? 1 : kRecheckTokens;
     while (static_cast<long long>(per_sweep) * num_centroids > 49152) per_sweep /= 2;
     const int smem = per_sweep * num_centroids * static_cast<int>(sizeof(float));
     if (head_dim == 128) {
@@ -842,7 +842,7 @@ int sqattn_kmeans_assign(const void* data, const void* centroids, int32_t dtype,
       if (bf16) SQ_CUDA(cudaFuncSetAttribute(kmeans_recheck_list_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       else SQ_CUDA(cudaFuncSetAttribute(kmeans_recheck_list_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     }
-    SQ_KM_DISPATCH(kmeans_recheck_list_kernel, <<<kGrid, 256, smem, stream>>>(d8, c8, idx, w.flagged, w.flagged_count, w.flagged_cap,
+    SQ_KM_DISPATCH(kmeans_recheck_list_kernel, <<<148 * 4, 256, smem, stream>>>(d8, c8, idx, w.flagged, w.flagged_count, w.flagged_cap,
                                                                              w.max_cnorm2, groups, num_tokens, num_centroids, per_sweep));
   }
   SQ_CUDA(cudaGetLastError());

@@ -226,7 +226,7 @@ def _exact_assignment(data, cent):
 @pytest.mark.parametrize("g,t,k,d,twice,zeros", [
     (2, 10000, 6144, 128, 64, 0), (1, 20000, 6176, 128, 64, 0), (2, 7000, 9600, 64, 4800, 0), (1, 10000, 12320, 128, 64, 0),
     (1, 5000, 24608, 128, 12304, 0), (1, 2500, 49152, 64, 64, 0), (1, 900, 12320, 128, 6160, 0), (2, 9000, 64, 128, 32, 4500),
-    (8, 30000, 64, 64, 8, 0), (8, 250, 1024, 128, 8, 0)])
+    (8, 30000, 64, 64, 8, 0), (8, 100000, 64, 64, 8, 0), (8, 250, 1024, 128, 8, 0)])
 def test_many_centroids_and_long_lists(g, t, k, d, twice, zeros):
     """Every number of tokens that a sweep of the re-scoring takes (8, 4, 2 and 1 as their scores' memory allows, 1 in small
     calls), up to the most centroids a group may have; ranks counted by CTAs and, above 8192 clusters, by warps; and more listed
